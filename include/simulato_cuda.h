@@ -46,7 +46,7 @@ extern "C" {
 #define SIMK_OPT_TMA 6          /* TMA-pipelined persistent column pass where the grid allows it (default 1) */
 #define SIMK_OPT_GRAPHS_CACHED 7 /* read-only: slice loops held as instantiated CUDA graphs */
 /* On the first fused scan of a grid shape and form, time one slice step of the actual transmission and propagator
- * for each column tile (2, 4, 8, and 16 at 256 x 256 with SIMK_OPT_PAIRED), with and without the TMA passes, then for
+ * for each column tile (2, 4, 8, and 16 at 256), with and without the TMA passes, then for
  * batch sizes up to what half of the free device memory holds, and use the fastest wherever SIMK_OPT_COL_TILE /
  * SIMK_OPT_BATCH are 0 (automatic) and TMA is allowed. The choice is kept per (grid, form) in the context. Default 0 (off). */
 #define SIMK_OPT_AUTOTUNE 8
@@ -72,14 +72,13 @@ extern "C" {
  * single GaussianGenerator stream over the samples and values in order (ScanOperations.swift:80-117), walked by one
  * device thread, so a seed gives the reference's draws. */
 #define SIMK_OPT_POISSON_STREAM 14
-/* The fused form's passes at lengths 3 or 5 times a power of two (384, 640, 768, 1536): 1 (default) = the composite
+/* The fused form's passes at lengths 3 or 5 times a power of two (192, 320, 384, 640, 768, 1536): 1 (default) = the
+ * two-pass engine (lengths up to 1024, column tiles of 8; one shared-memory exchange a transform), else the composite
  * register engine (each line as 3 or 5 register-resident power-of-two transforms of its decimated sub-lines); 0 = the
- * shared-memory Stockham engine. */
+ * shared-memory Stockham engine (384, 640, 768, 1536) or the runtime-plan kernels. */
 #define SIMK_OPT_COMPOSITE 15
-/* The fused form's column passes at grid sides 256, 512 and 1024: 1 (default) = tiles of 16 (256) or 8 columns, one
- * thread transforming the same rows of two adjacent columns, so that every global row segment is 128 or 64 bytes wide
- * (the pass then moves its bytes at close to the device's copy rate), where SIMK_OPT_COL_TILE is 0 or that width;
- * 0 = one column a thread, SIMK_OPT_COL_TILE (default 4) columns a tile. */
+/* Kept for callers: accepted and read back, but both values run the same kernels. (It chose between one and two columns
+ * a thread; the two-pass engine, which takes 8-column tiles where SIMK_OPT_COL_TILE is 0 or 8, 16 at 256, has one.) */
 #define SIMK_OPT_PAIRED 20
 /* read-only, the last fused simk_job_table_run: host launch calls that ran its slice steps (1: one CUDA graph launch,
  * with SIMK_OPT_GRAPHS on and SIMK_OPT_TIMING off), the kernels inside them, and the grid shapes they covered */

@@ -151,8 +151,8 @@ struct Context {
     int tcgen05 = 2;        // the bf16x3 form's DFT stages on tcgen05 where its tiles fit (else mma.sync): 2 stacked
     int epilogue_detect = 1;  // channel detectors summed in the last column pass (TMA passes)
     int poisson_stream = 0;   // Poisson noise: 0 = a generator per value and sample, 1 = the reference's one stream
-    int composite = 1;        // fused passes at 3 or 5 times a power of two: the composite register engine
-    int paired = 1;           // fused column passes at 256 and 512 on column pairs (engine 5)
+    int composite = 1;        // fused passes at 3 or 5 times a power of two: the two-pass or composite register engine
+    int paired = 1;           // SIMK_OPT_PAIRED, kept for callers: read back, chooses nothing
     // the last fused job table: host launch calls for its slice steps (1 when captured as one graph), the kernels in
     // them, and the grid shapes they covered
     long long table_launches = 0, table_kernels = 0;
@@ -179,6 +179,7 @@ struct Context {
     const int* wave_p = nullptr;
     int wave_p_blocks = 0;
     std::map<std::pair<int, int>, std::unique_ptr<LinePlan>> plans;
+    std::map<int, DeviceBuffer> twopass_tables;  // the two-pass engine's twiddles by line length
     std::map<std::tuple<int, int, double, double, double, double, double, double>, std::unique_ptr<Propagator>> props;
     // workspaces
     DeviceBuffer work_a, work_b, work_c, rx, ry, positions, partial;

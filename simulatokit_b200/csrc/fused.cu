@@ -19,6 +19,7 @@
 #include "tc5fft.cuh"
 #include "tcfft.cuh"
 #include "tma.cuh"
+#include "twopass.cuh"
 
 namespace simk {
 
@@ -314,78 +315,6 @@ __device__ __forceinline__ void ct_fft_from(float2 (&v)[8], unsigned t, const Tw
     }
 }
 
-// ---- column pairs (engine 5): one thread transforms the same rows of two adjacent columns -----------------------------
-// Thread (c, t) of a column tile eight columns wide holds columns 2c and 2c + 1 of rows t + T i: every load and store of
-// the tile moves both as one 16-byte access, and the exchanges keep the pair together in one float4 slot. Pair c's
-// exchange region is N float4 slots, slot s at swz(s) ^ 2c: a quarter warp (two t, four c) then reaches eight
-// different 16-byte bank groups in every scatter and gather of these plans (bit 0 of the swizzled slot tells the two t
-// apart, 2c the four pairs). The twiddles depend on t only, so both columns share them. `after_first_sync` runs right
-// after the first barrier of the transform (by then every thread has finished what preceded the transform).
-template <int N, int F, int DIR, typename Hook>
-__device__ __forceinline__ void ct2_fft_from(float2 (&v0)[8], float2 (&v1)[8], unsigned t, const TwRegs<N>& tr,
-                                             float4* __restrict__ region, int xc, Hook&& after_first_sync) {
-    using P = Pow2<N>;
-    if constexpr (F < P::NP) {
-        constexpr int R = P::radix(F), NS = P::ns(F), Q = 8 / R;
-        constexpr bool SC = (F + 1 < P::NP);
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            float2 a[R], b[R];
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                a[r] = v0[q + r * Q];
-                b[r] = v1[q + r * Q];
-            }
-            if constexpr (F > 0) {
-#pragma unroll
-                for (int r = 1; r < R; ++r) {
-                    const float2 w = tr.w[F - 1][q * (R - 1) + r - 1];
-                    a[r] = (DIR < 0) ? cmul(a[r], w) : cmulc(a[r], w);
-                    b[r] = (DIR < 0) ? cmul(b[r], w) : cmulc(b[r], w);
-                }
-            }
-            if constexpr (R == 2) {
-                bfly2<DIR>(a);
-                bfly2<DIR>(b);
-            } else if constexpr (R == 4) {
-                bfly4<DIR>(a);
-                bfly4<DIR>(b);
-            } else {
-                bfly8<DIR>(a);
-                bfly8<DIR>(b);
-            }
-            if constexpr (SC) {
-                const int jj = (int)t + P::T * q;
-                const int k = jj & (NS - 1);
-                const int o = (jj - k) * R + k;
-#pragma unroll
-                for (int r = 0; r < R; ++r) region[swz(o + r * NS) ^ xc] = make_float4(a[r].x, a[r].y, b[r].x, b[r].y);
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    v0[q + r * Q] = a[r];
-                    v1[q + r * Q] = b[r];
-                }
-            }
-        }
-        if constexpr (SC) {
-            __syncthreads();
-            if constexpr (F == 0) after_first_sync();
-            // as in ct_fft_from: swz(t + T i) ^ xc = (a ^ c_i) + T i with the per-thread a = swz(t) ^ xc (xc < 8 and
-            // swz(t) < T leave T i's bits alone)
-            const int a0 = ((int)t ^ (((int)t >> 3) & 15)) ^ xc;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float4 x = region[(a0 ^ (((P::T >> 3) * i) & 15)) + P::T * i];
-                v0[i] = make_float2(x.x, x.y);
-                v1[i] = make_float2(x.z, x.w);
-            }
-            __syncthreads();
-        }
-        ct2_fft_from<N, F + 1, DIR>(v0, v1, t, tr, region, xc, after_first_sync);
-    }
-}
-
 // ---- composite lengths N = R M (R = 3 or 5, M a power of two >= 64): the register engine on R sub-lines ---------------
 // A line's N / 8 threads form R sub-lines of TS = M / 8 threads; thread (g, u) is sub-line g, thread u. Decimation in
 // frequency from natural order (comp_dif_in, then the M-point register transform of each sub-line):
@@ -592,13 +521,12 @@ __device__ __forceinline__ void stage_wait(uint64_t* full, int s, int it, bool n
     }
 }
 
-// columns: tile = (wave b, TC columns from iy0); a stage holds the wave tile and the P tile, N x TC each (engine 5:
-// the wave tile only, beside one P buffer).
+// columns: tile = (wave b, TC columns from iy0); a stage holds the wave tile and the P tile, N x TC each.
 // Engines: 0 register-resident float32 Cooley-Tukey passes (powers of two); 1 radix-16 stages as mma.sync products of
 // split-BF16 operands on a shared-memory tile (tcfft.cuh, the bf16x3 form); 2 float32 shared-memory Stockham
 // (ccfft.cuh); 3 radix-16 stages as tcgen05.mma products (tc5fft.cuh, the bf16x3 form at 256 and 512); 4 the composite
-// register engine (lengths 3 or 5 times a power of two: R sub-lines of engine 0); 5 engine 0 on column pairs (8- or
-// 16-column tiles, two adjacent columns a thread; MODE 2 there generates the probes from their spectrum).
+// register engine (lengths 3 or 5 times a power of two: R sub-lines of engine 0). The two-pass engine, which takes most
+// lengths before these, has kernels of its own (twopass_kernels.cuh).
 // Height of the column pass's TMA boxes: the largest divisor of N that is at most 256 (the box limit).
 constexpr int tma_box_rows(int n) {
     for (int h = 256; h > 1; --h)
@@ -614,11 +542,11 @@ constexpr int rows_per_tile(int n, int max_threads = 256) {
 }
 constexpr int rows_tile(int n, int eng) { return rows_per_tile(n, eng == 4 ? 384 : 256); }
 
-// State an engine keeps per thread: register twiddles (0, 5), the DFT-16 fragments (1), nothing (2), the tcgen05 block
+// State an engine keeps per thread: register twiddles (0), the DFT-16 fragments (1), nothing (2), the tcgen05 block
 // state (3), the sub-lines' register twiddles (4).
 template <int N, int ENG>
 using EngineState = std::conditional_t<
-    ENG == 0 || ENG == 5, TwRegs<N>,
+    ENG == 0, TwRegs<N>,
     std::conditional_t<ENG == 1, Dft16Frags,
                        std::conditional_t<ENG == 3, Tc5, std::conditional_t<ENG == 4, TwRegs<CompPlan<N>::M>, int>>>>;
 
@@ -676,55 +604,42 @@ constexpr int tc_min_blocks(int threads, int eng) {
     if (eng == 1 || eng == 3) return threads <= 256 ? 2 : 1;
     if (eng == 0) return threads == 256 ? 3 : 1;
     if (eng == 4) return threads <= 256 ? 3 : (threads <= 384 ? 2 : 1);
-    if (eng == 5) return threads <= 256 ? 2 : 1;
     return 1;
 }
-// Threads across a column tile: one per column, or one per column pair (engine 5).
-constexpr int cols_tx(int tc, int eng) { return eng == 5 ? tc / 2 : tc; }
 
 template <int N, int TC, int MODE, int ENG>
-__global__ void __launch_bounds__(cols_tx(TC, ENG) * (N / 8), tc_min_blocks(cols_tx(TC, ENG) * (N / 8), ENG))
-    fused_cols_tma(const __grid_constant__ CUtensorMap map,
+__global__ void __launch_bounds__(TC * (N / 8), tc_min_blocks(TC * (N / 8), ENG)) fused_cols_tma(const __grid_constant__ CUtensorMap map,
                                                                const __grid_constant__ CUtensorMap pmap,
                                                                float2* __restrict__ psi, float pscale, int ny,
                                                                int count, const float2* __restrict__ tw, int* err,
                                                                const int* __restrict__ p_row, const DetectArgs det,
-                                                               int tc5_stack, const float2* __restrict__ rx,
-                                                               const float2* __restrict__ ry) {
+                                                               int tc5_stack) {
     extern __shared__ __align__(128) unsigned char smem_tma[];
     constexpr int T = N / 8;
     constexpr int BOXH = tma_box_rows(N);
     constexpr int NBOX = N / BOXH;
     constexpr int TILE = N * TC;  // float2 per tile
-    // engine 5: a stage holds only the wave tile and the P tile has one buffer of its own (refilled for the next tile
-    // once the multiply is done), so that two CTAs of eight-column tiles fit an SM
-    constexpr bool PSEP = (ENG == 5);
-    constexpr int TX = cols_tx(TC, ENG);
-    constexpr int SST = (PSEP ? 1 : 2) * TILE;  // float2 per stage
+    constexpr int SST = 2 * TILE;  // float2 per stage
     constexpr uint32_t STAGE_BYTES = (uint32_t)SST * sizeof(float2);
     __shared__ __align__(8) uint64_t full[2];
-    __shared__ __align__(8) uint64_t pfull;
     __shared__ int abort_flag;
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(8) uint64_t mma_bar;
-    __shared__ double red5[PSEP && MODE == 3 ? TX * T / 32 * 64 : 1];  // engine 5's detector sums (C <= 64)
     float2* stages = reinterpret_cast<float2*>(smem_tma);
-    [[maybe_unused]] float2* const ptile = stages + 2 * SST;  // engine 5's P tile (the spectrum's in MODE 2)
     const int c = threadIdx.x;
     const unsigned t = threadIdx.y;
-    const int tid = (int)t * TX + c;
+    const int tid = (int)t * TC + c;
     const unsigned tiles_per_wave = (unsigned)(ny / TC);
     const unsigned ntiles = (unsigned)count * tiles_per_wave;  // < 2^31: checked by the launcher
     if (tid == 0) {
         mbar_init(&full[0], 1);
         mbar_init(&full[1], 1);
-        mbar_init(&pfull, 1);
         fence_barrier_init();
         abort_flag = 0;
     }
     __syncthreads();
     [[maybe_unused]] EngineState<N, ENG> eng;
-    if constexpr (ENG == 0 || ENG == 5) tw_load<N, 1>(eng, t, tw);
+    if constexpr (ENG == 0) tw_load<N, 1>(eng, t, tw);
     else if constexpr (ENG == 4) tw_load<CompPlan<N>::M, 1, CompPlan<N>::R>(eng, t % CompPlan<N>::TS, tw);
     else if constexpr (ENG == 1) eng = dft16_frags(tid & 31);
     else if constexpr (ENG == 3)
@@ -735,35 +650,19 @@ __global__ void __launch_bounds__(cols_tx(TC, ENG) * (N / 8), tc_min_blocks(cols
         const int iy0 = (int)(tile - (unsigned)b * tiles_per_wave) * TC;
         float2* dst = stages + s * SST;
         const int prow = p_row ? p_row[b] * N : 0;  // job tables: this wave's propagator among the stacked ones
-        if constexpr (MODE == 2) {
-            mbar_arrive_expect_tx(&full[s], 0);  // probes: no wave to load, the phase completes at once
-            return;
-        }
         mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
 #pragma unroll
         for (int k = 0; k < NBOX; ++k) {
             tma_load_2d(dst + k * BOXH * TC, &map, &full[s], 2 * iy0, b * N + k * BOXH);
-            if constexpr (!PSEP) tma_load_2d(dst + TILE + k * BOXH * TC, &pmap, &full[s], 2 * iy0, prow + k * BOXH);
+            tma_load_2d(dst + TILE + k * BOXH * TC, &pmap, &full[s], 2 * iy0, prow + k * BOXH);
         }
     };
-    // engine 5: the P tile of `tile` into its own buffer, completing on pfull (one phase per tile)
-    [[maybe_unused]] auto issue_p = [&](unsigned tile) {
-        const int b = (int)(tile / tiles_per_wave);
-        const int iy0 = (int)(tile - (unsigned)b * tiles_per_wave) * TC;
-        const int prow = (MODE != 2 && p_row) ? p_row[b] * N : 0;
-        mbar_arrive_expect_tx(&pfull, (uint32_t)TILE * sizeof(float2));
-#pragma unroll
-        for (int k = 0; k < NBOX; ++k) tma_load_2d(ptile + k * BOXH * TC, &pmap, &pfull, 2 * iy0, prow + k * BOXH);
-    };
     unsigned tile = blockIdx.x;
-    if (tid == 0 && tile < ntiles) {
-        issue(tile, 0);
-        if constexpr (PSEP) issue_p(tile);
-    }
+    if (tid == 0 && tile < ntiles) issue(tile, 0);
     for (int it = 0; tile < ntiles; tile += gridDim.x, ++it) {
         const int s = it & 1;
         float2* buf = stages + s * SST;
-        const float2* pbuf = PSEP ? ptile : buf + TILE;
+        const float2* pbuf = buf + TILE;
         const unsigned next = tile + gridDim.x;
         if (tid == 0) {
             // the previous tile's TMA store must have read its shared-memory source (a stage or the scratch tile)
@@ -773,15 +672,6 @@ __global__ void __launch_bounds__(cols_tx(TC, ENG) * (N / 8), tc_min_blocks(cols
             const bool more = !abort_flag && next < ntiles;
             if (more) issue(next, s ^ 1);
             stage_wait(full, s, it, more, err, &abort_flag);
-            if constexpr (PSEP) {
-                // this tile's P, issued at the start or once the previous tile's multiply was done; waited for after
-                // an abandoned wave copy too, so that no copy is in flight when the block leaves
-                if (!mbar_wait_bounded(&pfull, (uint32_t)(it & 1))) {
-                    atomicExch(err, 1);
-                    if (!abort_flag && more) mbar_wait_bounded(&full[s ^ 1], (uint32_t)(((it + 1) >> 1) & 1));
-                    abort_flag = 1;
-                }
-            }
         }
         __syncthreads();
         if (abort_flag) break;
@@ -802,55 +692,6 @@ __global__ void __launch_bounds__(cols_tx(TC, ENG) * (N / 8), tc_min_blocks(cols
             // thread 0 stores the tile with TMA after the barrier below
 #pragma unroll
             for (int i = 0; i < 8; ++i) buf[(t + T * i) * TC + c] = v[i];
-            store_src = buf;
-        } else if constexpr (ENG == 5) {
-            // column pairs: thread (c, t) holds columns 2c, 2c + 1 of rows t + T i (one 16-byte access per row)
-            static_assert(TX == 4 || TX == 8, "column pairs: four or eight pairs a tile");
-            float4* const tile4 = reinterpret_cast<float4*>(buf);
-            const float4* const p4 = reinterpret_cast<const float4*>(pbuf);
-            float4* const region = tile4 + c * N;
-            // the slot XOR that spreads a quarter warp (two t and four pairs, or one t and eight) over the bank groups
-            const int xc = (TX == 4) ? 2 * c : c;
-            // behind the first barrier of the transform that follows the last read of the P buffer, every thread has
-            // read it: the next tile's P (or spectrum) may come
-            auto next_p = [&] {
-                if (tid == 0 && !abort_flag && next < ntiles) issue_p(next);
-            };
-            float2 v0[8], v1[8];
-            if constexpr (MODE == 2) {
-                // probes: the spectrum tile (in the P buffer) times the shift ramps r_x[ix] r_y[iy] of wave b, then the
-                // inverse transform; nothing is read from the stage
-                const int col = iy + c;  // iy - c + 2 c: the pair's first column
-                const float2 ry0 = __ldg(ry + (size_t)b * ny + col), ry1 = __ldg(ry + (size_t)b * ny + col + 1);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int ix = (int)t + T * i;
-                    const float4 sp = p4[ix * TX + c];
-                    const float2 r = __ldg(rx + (size_t)b * N + ix);
-                    v0[i] = cmul(cmul(make_float2(sp.x, sp.y), r), ry0);
-                    v1[i] = cmul(cmul(make_float2(sp.z, sp.w), r), ry1);
-                }
-                ct2_fft_from<N, 0, +1>(v0, v1, t, eng, region, xc, next_p);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float4 x = tile4[(t + T * i) * TX + c];
-                    v0[i] = make_float2(x.x, x.y);
-                    v1[i] = make_float2(x.z, x.w);
-                }
-                __syncthreads();  // the wave tile has been read: it becomes the pairs' exchange regions
-                ct2_fft_from<N, 0, -1>(v0, v1, t, eng, region, xc, [] {});
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float4 pp = p4[(t + T * i) * TX + c];
-                    v0[i] = cmul(v0[i], make_float2(pp.x, pp.y)) * pscale;
-                    v1[i] = cmul(v1[i], make_float2(pp.z, pp.w)) * pscale;
-                }
-                if constexpr (MODE == 0) ct2_fft_from<N, 0, +1>(v0, v1, t, eng, region, xc, next_p);
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                tile4[(t + T * i) * TX + c] = make_float4(v0[i].x, v0[i].y, v1[i].x, v1[i].y);
             store_src = buf;
         } else if constexpr (ENG == 4) {
             // composite length: R sub-lines of TS threads per column; a sub-line's exchanges use its own part of the
@@ -945,16 +786,11 @@ __global__ void __launch_bounds__(cols_tx(TC, ENG) * (N / 8), tc_min_blocks(cols
             for (int k = 0; k < NBOX; ++k) tma_store_2d(&map, store_src + k * BOXH * TC, 2 * iy0, b * N + k * BOXH);
             bulk_commit();
         }
-        if constexpr (PSEP && MODE != 0 && MODE != 2) {
-            // without an inverse transform the P tile is free from the barrier above on
-            if (tid == 0 && !abort_flag && next < ntiles) issue_p(next);
-        }
         if constexpr (MODE == 3) {
             // the tile the result is not in holds the warps' sums (TILE float2 >= NT / 32 * C doubles, C <= 64): the P
-            // tile (read by now), or for the composite engine, whose result is in the P tile, the wave tile; engine 5,
-            // whose P buffer is being refilled, has an array of its own
-            double* sums = PSEP ? red5 : reinterpret_cast<double*>((ENG == 4) ? buf : buf + TILE);
-            detect_tile<TX * T>(store_src, det, b, (iy - c) / TC, tid, sums);
+            // tile (read by now), or for the composite engine, whose result is in the P tile, the wave tile
+            double* sums = reinterpret_cast<double*>((ENG == 4) ? buf : buf + TILE);
+            detect_tile<TC * T>(store_src, det, b, (iy - c) / TC, tid, sums);
             fence_proxy_async_shared();  // the sums were written by this proxy; the next copy into the stage by TMA
             __syncthreads();  // the partials' reads of the tile and of the sums precede the next copy into the stage
         }
@@ -1246,11 +1082,12 @@ RegChoice choose(int n) {
 
 RegPlan reg_plan(Context& ctx, int n) {
     RegChoice ch = choose(n);
-    SIMK_REQUIRE(ch.E != 0, "no register FFT plan for length " + std::to_string(n));
+    SIMK_REQUIRE(ch.E != 0 || (ctx.tma && twopass_length(n)), "no register FFT plan for length " + std::to_string(n));
+    if (twopass_length(n)) twopass_table(ctx, n);  // created here, before a capture
     RegPlan p{};
     p.n = n;
-    p.E = ch.E;
-    p.T = n / ch.E;
+    p.E = ch.E;  // 0: only the two-pass engine takes the length
+    p.T = ch.E ? n / ch.E : 0;
     p.npass = (int)ch.fac.size();
     for (int i = 0; i < p.npass; ++i) p.fac[i] = ch.fac[i];
     p.tw = static_cast<const float2*>(ctx.plan(n, 32).tw.ptr);
@@ -1347,7 +1184,6 @@ void ensure_err_flag(Context& ctx) {
 // tile (1, 2) or the tcgen05 engine's operands (3).
 constexpr size_t tma_pass_smem(int n, int lines, int eng) {
     return eng == 3   ? 4 * (size_t)n * lines * sizeof(float2) + tc5_smem_bytes(tc5_blocks(n, lines))
-           : eng == 5 ? 3 * (size_t)n * lines * sizeof(float2)  // two wave stages and one P tile
                       : (eng != 0 && eng != 4 ? 5 : 4) * (size_t)n * lines * sizeof(float2);
 }
 
@@ -1442,19 +1278,16 @@ bool launch_cols_tma_m(Context& ctx, const RegPlan& p, const ColArgs& a, int cou
     if (occupancy < 0) {
         SIMK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         SIMK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-        SIMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occupancy, kern, cols_tx(TC, ENG) * T, smem));
-        occupancy = std::max(occupancy, fitting_blocks((const void*)kern, cols_tx(TC, ENG) * T, smem, ctx.device));
+        SIMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occupancy, kern, TC * T, smem));
+        occupancy = std::max(occupancy, fitting_blocks((const void*)kern, TC * T, smem, ctx.device));
     }
     const int stack = ctx.tcgen05 == 2 ? 1 : 0;
     const int blocks_per_sm = pass_blocks_per_sm(occupancy, ENG, ENG == 3 ? tc5_blocks(N, TC) : 0, stack != 0);
     if (blocks_per_sm <= 0) return false;
     ensure_err_flag(ctx);
     const CUtensorMap map = encode_tensor_map_2d(a.psi, 2ULL * a.ny, (unsigned long long)count * N, 2 * TC, BOXH);
-    // the P tiles, or for the probes (MODE 2) the spectrum's
-    const CUtensorMap pmap =
-        MODE == 2 ? encode_tensor_map_2d(const_cast<float2*>(a.spectrum), 2ULL * a.ny, (unsigned long long)N, 2 * TC, BOXH)
-                  : encode_tensor_map_2d(const_cast<float2*>(a.P), 2ULL * a.ny,
-                                         (unsigned long long)std::max(1, a.p_blocks) * N, 2 * TC, BOXH);
+    const CUtensorMap pmap = encode_tensor_map_2d(const_cast<float2*>(a.P), 2ULL * a.ny,
+                                                  (unsigned long long)std::max(1, a.p_blocks) * N, 2 * TC, BOXH);
     const long long ntiles = (long long)count * (a.ny / TC);
     if (ntiles >= (1LL << 31)) return false;
     DetectArgs det{};
@@ -1469,8 +1302,8 @@ bool launch_cols_tma_m(Context& ctx, const RegPlan& p, const ColArgs& a, int cou
         if (a.det_groups) *a.det_groups = tch.groups;
     }
     const int grid = (int)std::min<long long>(ntiles, (long long)blocks_per_sm * ctx.sm_count);
-    kern<<<grid, dim3(cols_tx(TC, ENG), T), smem, ctx.stream>>>(map, pmap, a.psi, a.pscale, a.ny, count, p.tw,
-                                                  ctx.err_flag.as<int>(), a.p_row, det, stack, a.rx, a.ry);
+    kern<<<grid, dim3(TC, T), smem, ctx.stream>>>(map, pmap, a.psi, a.pscale, a.ny, count, p.tw,
+                                                  ctx.err_flag.as<int>(), a.p_row, det, stack);
     SIMK_CUDA(cudaGetLastError());
     ++ctx.launches;
     return true;
@@ -1483,9 +1316,6 @@ bool launch_cols_tma(Context& ctx, const RegPlan& p, const ColArgs& a, int count
     if (a.mode == 0) return launch_cols_tma_m<N, TC, 0, ENG>(ctx, p, a, count);
     if (a.mode == 1) return launch_cols_tma_m<N, TC, 1, ENG>(ctx, p, a, count);
     if (a.mode == 3) return launch_cols_tma_m<N, TC, 3, ENG>(ctx, p, a, count);
-    if constexpr (ENG == 5) {
-        if (a.mode == 2) return launch_cols_tma_m<N, TC, 2, ENG>(ctx, p, a, count);  // probes from their spectrum
-    }
     return false;
 }
 
@@ -1501,15 +1331,8 @@ void launch_cols_ct(Context& ctx, const RegPlan& p, const ColArgs& a, int count)
 bool rows_ct(Context& ctx, const RegPlan& p, float2* psi, const float2* tmul, int nx, long long nrows, int inv, int fwd,
              float scale) {
     if (ctx.tma) {
-        bool done = false;
-        switch (p.n) {
-            case 256: done = launch_rows_tma<256, 0>(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale); break;
-            case 512: done = launch_rows_tma<512, 0>(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale); break;
-            case 1024: done = launch_rows_tma<1024, 0>(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale); break;
-            case 2048: done = launch_rows_tma<2048, 0>(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale); break;
-            default: break;
-        }
-        if (done) return true;
+        // (the two-pass engine has taken the shorter lengths)
+        if (p.n == 2048 && launch_rows_tma<2048, 0>(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale)) return true;
     }
     switch (p.n) {
         case 128: launch_rows_ct<128>(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale); return true;
@@ -1525,14 +1348,6 @@ template <int N>
 bool cols_ct_tc(Context& ctx, const RegPlan& p, const ColArgs& a, int count, int tc) {
     // TC x N/8 threads per CTA, at most 1024
     if (tc * (N / 8) > 1024 || a.ny % tc) return false;
-    // column pairs (engine 5, every mode including the probes' generation): tiles of 8 columns at 512 and 1024 (one
-    // 512-thread CTA an SM there) and 16 at 256, where the column tile is automatic or that
-    if constexpr (N == 512 || N == 256 || N == 1024) {
-        constexpr int TP = (N == 256) ? 16 : 8;
-        if (ctx.tma && ctx.paired && (ctx.col_tile == 0 || ctx.col_tile == TP) && a.ny % TP == 0 &&
-            launch_cols_tma<N, TP, 5>(ctx, p, a, count))
-            return true;
-    }
     if (ctx.tma && a.mode != 2) {
         switch (tc) {
             case 2: if (launch_cols_tma<N, 2>(ctx, p, a, count)) return true; break;
@@ -1639,7 +1454,7 @@ bool cols_tc(Context& ctx, const RegPlan& p, const ColArgs& a, int count) {
 template <int N>
 bool rows_cc_n(Context& ctx, const RegPlan& p, float2* psi, const float2* tmul, int nx, long long nrows, int inv,
                int fwd, float scale) {
-    if constexpr (comp_length(N)) {
+    if constexpr (comp_length(N) && N > 1024) {  // (the two-pass engine has taken the shorter lengths)
         if (ctx.composite && launch_rows_tma<N, 4>(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale)) return true;
     }
     return launch_rows_tma<N, 2>(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale);
@@ -1692,6 +1507,52 @@ bool cols_cc(Context& ctx, const RegPlan& p, const ColArgs& a, int count) {
     }
 }
 
+// ---- the two-pass engine (twopass.cuh): one exchange a transform, wherever the length has a plan and the settings ask
+// for no other engine. Measured against the engines it replaced (one box, us a launch, rows | columns): 512^2 x 512 waves
+// 516 -> 420 | 488 -> 440; 1024^2 x 128 671 -> 438 | 735 -> 556; 768^2 x 64 249 -> 148 | 246 -> 166; 500^2 x 144
+// 691 -> 166 | 632 -> 170; 256^2 x 256 69 -> 52 | 68 -> 62 --------------------------------------------------------------
+bool two_wanted(const Context& ctx, int n) {
+    if (!ctx.tma || !twopass_length(n)) return false;
+    return comp_length(n) ? ctx.composite != 0 : true;
+}
+
+bool rows_two(Context& ctx, const RegPlan& p, float2* psi, const float2* tmul, int nx, long long nrows, int inv, int fwd,
+              float scale) {
+    return two_wanted(ctx, p.n) && twopass_rows(ctx, psi, tmul, nx, p.n, nrows, inv, fwd, scale);
+}
+
+// The column tile (SIMK_OPT_COL_TILE) that names it beside 0: its tiles are 8 columns wide; at 256, where 8 names the
+// register engine's tile, 16 does.
+int two_tile(int n) { return n == 256 ? 16 : 8; }
+
+// Columns of 128 points stay on the register engine: its 4-column tiles took 41.5 us for 512 waves and 7.0 us for one,
+// the two-pass engine 45.2 and 8.5 (at 192 points 74.9 against the runtime plan's several times that; at 256 61.8
+// against 68.3 for 256 waves).
+bool cols_two_wanted(const Context& ctx, int n) {
+    return n > 128 && two_wanted(ctx, n) && (ctx.col_tile == 0 || ctx.col_tile == two_tile(n));
+}
+
+bool cols_two(Context& ctx, const RegPlan& p, const ColArgs& a, int count) {
+    if (!cols_two_wanted(ctx, p.n)) return false;
+    ensure_err_flag(ctx);
+    TwoPassCols c;
+    c.psi = a.psi;
+    c.P = a.P;
+    c.pscale = a.pscale;
+    c.mode = a.mode;
+    c.ny = a.ny;
+    c.count = count;
+    c.spectrum = a.spectrum;
+    c.rx = a.rx;
+    c.ry = a.ry;
+    c.p_row = a.p_row;
+    c.det = &a.det;
+    int groups = 0;
+    if (!twopass_cols(ctx, p.n, c, &groups)) return false;
+    if (a.mode == 3 && a.det_groups) *a.det_groups = groups;
+    return true;
+}
+
 bool tc_length(int n) { return n == 256 || n == 512 || n == 768 || n == 1024 || n == 2048; }
 
 void launch_rows(Context& ctx, const RegPlan& p, float2* psi, const float2* tmul, int nx, long long nrows, int inv,
@@ -1702,6 +1563,7 @@ void launch_rows(Context& ctx, const RegPlan& p, float2* psi, const float2* tmul
             throw Error(SIMK_ERR_INVALID, "the bf16x3 form has no row pass for length " + std::to_string(p.n));
         return;
     }
+    if (rows_two(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale)) return;
     if (rows_ct(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale)) return;
     if (ctx.tma && rows_cc(ctx, p, psi, tmul, nx, nrows, inv, fwd, scale)) return;
     switch (p.E) {
@@ -1728,7 +1590,7 @@ int launch_cols(Context& ctx, const RegPlan& p, const ColArgs& a_in, int count) 
     if (a.mode == 3) {
         a.det_groups = &groups;
         const bool done = ctx.form == SIMK_FORM_BF16X3 ? cols_tc(ctx, p, a, count)
-                                                       : (cols_ct(ctx, p, a, count) ||
+                                                       : (cols_two(ctx, p, a, count) || cols_ct(ctx, p, a, count) ||
                                                           (ctx.tma && cols_cc(ctx, p, a, count)));
         if (done) return groups;
         a.mode = 1;
@@ -1739,6 +1601,7 @@ int launch_cols(Context& ctx, const RegPlan& p, const ColArgs& a_in, int count) 
             throw Error(SIMK_ERR_INVALID, "the bf16x3 form has no column pass for length " + std::to_string(p.n));
         return 0;
     }
+    if (cols_two(ctx, p, a, count)) return 0;
     if (cols_ct(ctx, p, a, count)) return 0;
     if (ctx.tma && a.mode != 2 && cols_cc(ctx, p, a, count)) return 0;
     switch (p.E) {
@@ -1787,7 +1650,7 @@ bool fused_supported(Context& ctx, const GridGeom& g) {
         SIMK_REQUIRE(ctx.tma, "the bf16x3 form runs on the TMA-pipelined passes (SIMK_OPT_TMA must be on)");
         return true;
     }
-    return choose(g.nx).E != 0 && choose(g.ny).E != 0;
+    return (choose(g.nx).E != 0 || cols_two_wanted(ctx, g.nx)) && (choose(g.ny).E != 0 || two_wanted(ctx, g.ny));
 }
 
 namespace {
@@ -1822,8 +1685,7 @@ int propagate_fused(Context& ctx, PotentialImpl& pot, double energy, double tx, 
     key_append(key, kspace_last);
     key_append(key, ctx.form);
     key_append(key, ctx.col_tile);
-    key_append(key, ctx.paired);
-    key_append(key, ctx.tma);
+      key_append(key, ctx.tma);
     key_append(key, ctx.tcgen05);
     key_append(key, ctx.composite);
     key_append(key, ctx.stream);
@@ -1991,6 +1853,7 @@ Context::Tuned autotune(Context& ctx, PotentialImpl& pot, double energy, double 
     // the engines to choose from: the composite register engine or the shared-memory one (fused form, lengths 3 or 5
     // times a power of two), the tcgen05 engine's two product orders or the mma.sync engine (bf16x3 form, 256, 512)
     std::vector<int> engines{-1};
+    const bool two_side = twopass_length(g.nx) && g.nx > 128;
     const bool comp_side = comp_length(g.nx) || comp_length(g.ny);
     const bool tc5_side = (g.nx == 256 || g.nx == 512) && (g.ny == 256 || g.ny == 512);
     if (ctx.form == SIMK_FORM_FUSED && comp_side) engines = {1, 0};
@@ -2033,10 +1896,13 @@ Context::Tuned autotune(Context& ctx, PotentialImpl& pot, double energy, double 
                 if (tma && !save_tma) continue;
                 if (!tma && ctx.form == SIMK_FORM_BF16X3) continue;  // the tensor-core form runs on the TMA passes only
                 if (!tma && eng == 0 && ctx.form == SIMK_FORM_FUSED) continue;  // the engines differ on TMA passes only
+                // lengths that only the two-pass engine takes: neither without the TMA passes nor at other widths
+                const bool cols_only_two = choose(g.nx).E == 0;
+                if (!tma && (cols_only_two || choose(g.ny).E == 0)) continue;
                 for (int tc : {2, 4, 8, 16}) {
-                    if (g.ny % tc || tc * (g.nx / 8) > 1024) continue;
-                    // 16 columns only where the column pairs take them (256^2)
-                    if (tc == 16 && !(ctx.paired && g.nx == 256 && ctx.form == SIMK_FORM_FUSED && tma)) continue;
+                    // the two-pass engine's tiles are 8 columns wide (the last may be narrower), whatever the other side
+                    const bool two = tma && tc == two_tile(g.nx) && ctx.form == SIMK_FORM_FUSED && eng != 0 && two_side;
+                    if (!two && (tc == 16 || cols_only_two || g.ny % tc || tc * (g.nx / 8) > 1024)) continue;
                     ctx.tma = tma;
                     ctx.col_tile = tc;
                     const double t = time_per_wave(b0);
@@ -2230,7 +2096,7 @@ struct TableCache {
 std::string table_key(const Context& ctx, const std::vector<JobSpec>& jobs) {
     std::string k;
     auto add = [&](const void* p, size_t n) { k.append(static_cast<const char*>(p), n); };
-    const int opts[] = {ctx.form, ctx.tma, ctx.col_tile, ctx.composite, ctx.tcgen05, ctx.paired};
+    const int opts[] = {ctx.form, ctx.tma, ctx.col_tile, ctx.composite, ctx.tcgen05};
     add(opts, sizeof(opts));
     for (const JobSpec& j : jobs) {
         const void* ids[] = {j.pot, j.pot->t.ptr};

@@ -932,10 +932,10 @@ std::unique_ptr<DetectorPlan> build_detector_plan(Context& ctx, const GridGeom& 
 const DetectorPlan::TileChannels& DetectorPlan::tiles(int tc) {
     for (auto& t : tile_channels)
         if (t->tc == tc) return *t;
-    SIMK_REQUIRE(tc >= 1 && grid_ny % tc == 0, "column tile width must divide the grid");
+    SIMK_REQUIRE(tc >= 1, "column tile width must be positive");
     auto t = std::make_unique<TileChannels>();
     t->tc = tc;
-    t->groups = grid_ny / tc;
+    t->groups = (grid_ny + tc - 1) / tc;  // the last group may be narrower
     const int C = n_channels, G = t->groups;
     std::vector<std::vector<std::pair<int, float>>> lists((size_t)G * C);
     for (int ch = 0; ch < C; ++ch)

@@ -1,0 +1,32 @@
+// twopass.cuh -- the fused passes with one shared-memory exchange per transform (engine 6): what fused.cu calls. The
+// kernels are in twopass_kernels.cuh, instantiated by twopass_*.cu; the lengths are listed in twopass_plans.inc.
+#pragma once
+
+#include "context.cuh"
+
+namespace simk {
+
+struct TwoPassCols {
+    float2* psi = nullptr;
+    const float2* P = nullptr;
+    float pscale = 1.0f;
+    int mode = 0;  // 0: FFT, x P, IFFT; 1: FFT, x P; 2: the probes' spectrum, IFFT; 3: as 1, with the detection
+    int ny = 0, count = 0;
+    const float2* spectrum = nullptr;
+    const float2* rx = nullptr;
+    const float2* ry = nullptr;
+    const int* p_row = nullptr;  // job tables: wave b uses the propagator P + p_row[b] N
+    const FusedDetect* det = nullptr;
+};
+
+// Whether lines of n points have a plan here.
+bool twopass_length(int n);
+// The plan's twiddle table of n, created on first use (allocates and copies: not inside a stream capture).
+const float2* twopass_table(Context& ctx, int n);
+// The row pass over nrows = count nx rows of ny points: [inverse], x t x scale, [forward]. False: no plan for ny.
+bool twopass_rows(Context& ctx, float2* psi, const float2* tmul, int nx, int ny, long long nrows, int inv, int fwd,
+                  float scale);
+// The column pass over lines of nx points; with mode 3 *groups receives the column groups of the partial sums.
+bool twopass_cols(Context& ctx, int nx, const TwoPassCols& a, int* groups);
+
+}  // namespace simk

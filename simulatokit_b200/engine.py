@@ -24,11 +24,10 @@ class ExecutionOptions:
     (tcgen05.mma, tensor-memory accumulators) at grid sides 256 and 512: 2 (default) six stacked products a stage,
     1 twelve products of N = 32, 0 / False the warp-level mma.sync stages.
     epilogue_detect: sum the channel detectors inside the last column pass (TMA passes) instead of separate kernels.
-    composite: at grid sides 3 or 5 times a power of two (384, 640, 768, 1536) the fused passes transform each line as
-    register-resident power-of-two transforms of its decimated sub-lines; False keeps the shared-memory Stockham
-    engine. paired: at grid sides 512, 1024 and 256 the fused column pass takes tiles of 8 or 16 columns, one thread
-    per pair of adjacent columns (64- and 128-byte row segments in HBM), where col_tile is 0 or that width; False
-    keeps one column a thread."""
+    composite: at grid sides 3 or 5 times a power of two (192, 320, 384, 640, 768, 1536) the fused passes run on the
+    two-pass engine (one shared-memory exchange a transform; up to 1024) or the composite register engine; False keeps
+    the shared-memory Stockham engine. col_tile names it as 0 or 8 (16 at 256); other widths keep
+    the register engines. paired: accepted for callers that set it; both values run the same kernels."""
 
     FORMS = {"plain": L.FORM_PLAIN, "fused": L.FORM_FUSED, "bf16x3": L.FORM_BF16X3}
 

@@ -179,6 +179,8 @@ struct Context {
     const int* wave_p = nullptr;
     int wave_p_blocks = 0;
     std::map<std::pair<int, int>, std::unique_ptr<LinePlan>> plans;
+    DeviceBuffer lobato_elements;  // the scaled Lobato parameters of Z = 1 .. 103
+    DeviceBuffer evaluate_work;    // the surrogate's queries, their full projections and results
     std::map<int, DeviceBuffer> twopass_tables;  // the two-pass engine's twiddles by line length
     std::map<std::tuple<int, int, double, double, double, double, double, double>, std::unique_ptr<Propagator>> props;
     // workspaces

@@ -44,6 +44,10 @@ FiniteSetup finite_setup(const GridGeom& g, const std::vector<double>& dz, int n
 FiniteDevice upload_finite(Context& ctx, const FiniteSetup& s, DeviceBuffer& pairs, DeviceBuffer& ab,
                            DeviceBuffer& rmin, DeviceBuffer& rcut);
 void finite_profiles_quadrature(Context& ctx, const FiniteDevice& d, long long npairs, int nr, double* table);
+// The full projection P_inf(rho) = 2 sum_i [2 A_i/B_i K0(B_i rho) + A_i rho K1(B_i rho)] at n points (atomic number 1 to
+// 103, rho > 0), float64: on device arrays, or from and to the host.
+void infinite_points(Context& ctx, int n, const int* z_dev, const double* rho_dev, double* out_dev);
+std::vector<double> infinite_profiles(Context& ctx, const std::vector<int>& z, const std::vector<double>& rho);
 void finite_points(Context& ctx, const ElementAB* ab_dev, int n, const int* elem_dev, const double* rho_dev,
                    const double* zl_dev, const double* zu_dev, double* out_dev);
 void finite_splat(Context& ctx, PotentialImpl& pot, const FiniteSetup& s, const FiniteDevice& d, int nr,

@@ -545,14 +545,6 @@ __global__ void __launch_bounds__(kTcWarps * 32) k_sg_infer(const float* __restr
 }
 
 // ---- host --------------------------------------------------------------------------------------------------------
-double infinite_profile(int z, double rho) {
-    const ElementAB e = element_ab(z);
-    double s = 0.0;
-    for (int t = 0; t < 5; ++t)
-        s += 2.0 * e.A[t] / e.B[t] * std::cyl_bessel_k(0.0, e.B[t] * rho) + e.A[t] * rho * std::cyl_bessel_k(1.0, e.B[t] * rho);
-    return 2.0 * s;
-}
-
 namespace {
 
 struct Batch {  // a doubled batch: rows b (upper edge) and B + b (lower edge); per-block gradient rows
@@ -723,12 +715,13 @@ std::unique_ptr<SurrogateImpl> surrogate_train(Context& ctx, const std::vector<i
             surrogate_quadrature_points(ctx, z, rho, zl, zu, P.as<double>());
             std::vector<double> hp(m);
             SIMK_CUDA(cudaMemcpy(hp.data(), P.ptr, m * sizeof(double), cudaMemcpyDeviceToHost));
+            const std::vector<double> full = infinite_profiles(ctx, z, rho);
             for (int i = 0; i < m; ++i) {
                 all_z[first + i] = z[i];
                 all_rho[first + i] = rho[i];
                 all_zl[first + i] = zl[i];
                 all_zu[first + i] = zu[i];
-                all_F[first + i] = (float)(hp[i] / infinite_profile(z[i], rho[i]));
+                all_F[first + i] = (float)(hp[i] / full[i]);
             }
         }
     }
@@ -777,9 +770,10 @@ std::unique_ptr<SurrogateImpl> surrogate_train(Context& ctx, const std::vector<i
     surrogate_quadrature_points(ctx, z, rho, zl, zu, dq.as<double>());
     SIMK_CUDA(cudaMemcpy(q.data(), dq.ptr, 4096 * sizeof(double), cudaMemcpyDeviceToHost));
     surrogate_evaluate(ctx, *s, z, rho, zl, zu, e.data());
+    const std::vector<double> full = infinite_profiles(ctx, z, rho);
     double mx = 0.0, rms = 0.0;
     for (int i = 0; i < 4096; ++i) {
-        const double r = std::fabs(e[i] - q[i]) / infinite_profile(z[i], rho[i]);
+        const double r = std::fabs(e[i] - q[i]) / full[i];
         mx = std::max(mx, r);
         rms += r * r;
     }
@@ -793,22 +787,22 @@ void surrogate_evaluate(Context& ctx, const SurrogateImpl& s, const std::vector<
     const int n = (int)z.size();
     if (n == 0) return;
     set_infer_smem();
-    std::vector<double> pinf(n);
-    for (int i = 0; i < n; ++i) pinf[i] = infinite_profile(z[i], rho[i]);
-    DeviceBuffer dz(n * sizeof(int)), dr(n * sizeof(double)), dl(n * sizeof(double)), du(n * sizeof(double)),
-        dp(n * sizeof(double)), dout(n * sizeof(double));
-    SIMK_CUDA(cudaMemcpy(dz.ptr, z.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(dr.ptr, rho.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(dl.ptr, zl.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(du.ptr, zu.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(dp.ptr, pinf.data(), n * sizeof(double), cudaMemcpyHostToDevice));
+    // one buffer kept in the context: rho, zl, zu, the full projections, the results, the atomic numbers
+    ctx.evaluate_work.ensure((size_t)n * (5 * sizeof(double) + sizeof(int)));
+    double* const dr = ctx.evaluate_work.as<double>();
+    double *const dl = dr + n, *const du = dl + n, *const dp = du + n, *const dout = dp + n;
+    int* const dz = reinterpret_cast<int*>(dout + n);
+    SIMK_CUDA(cudaMemcpyAsync(dz, z.data(), n * sizeof(int), cudaMemcpyHostToDevice, ctx.stream));
+    SIMK_CUDA(cudaMemcpyAsync(dr, rho.data(), n * sizeof(double), cudaMemcpyHostToDevice, ctx.stream));
+    SIMK_CUDA(cudaMemcpyAsync(dl, zl.data(), n * sizeof(double), cudaMemcpyHostToDevice, ctx.stream));
+    SIMK_CUDA(cudaMemcpyAsync(du, zu.data(), n * sizeof(double), cudaMemcpyHostToDevice, ctx.stream));
+    infinite_points(ctx, n, dz, dr, dp);
     SgQueryPairs q{};
     k_sg_infer<false><<<infer_blocks(ctx, n), kTcWarps * 32, kTcSmem, ctx.stream>>>(
-        s.params.as<float>(), q, dz.as<int>(), dr.as<double>(), dl.as<double>(), du.as<double>(),
-        dp.as<double>(), n, dout.as<double>());
+        s.params.as<float>(), q, dz, dr, dl, du, dp, n, dout);
     SIMK_CUDA(cudaGetLastError());
     ++ctx.launches;
-    SIMK_CUDA(cudaMemcpyAsync(out_host, dout.ptr, n * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
+    SIMK_CUDA(cudaMemcpyAsync(out_host, dout, n * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
     SIMK_CUDA(cudaStreamSynchronize(ctx.stream));
 }
 

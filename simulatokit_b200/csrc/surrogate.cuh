@@ -40,7 +40,5 @@ void surrogate_profiles(Context& ctx, const SurrogateImpl& s, const FiniteDevice
 double surrogate_gradients(Context& ctx, SurrogateImpl& s, const std::vector<int>& z, const std::vector<double>& rho,
                            const std::vector<double>& zl, const std::vector<double>& zu,
                            const std::vector<double>& target, float* grads_host);
-// The analytic infinite projection 2 sum_i [2 A_i/B_i K0(B_i rho) + A_i rho K1(B_i rho)] (host, float64).
-double infinite_profile(int z, double rho);
 
 }  // namespace simk

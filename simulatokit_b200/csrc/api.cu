@@ -102,6 +102,7 @@ int simk_context_create(int32_t device, simk_context** out) {
             throw;
         }
         c->impl.stream = c->impl.own_stream;
+        device_context_made(device);
         *out = c;
     });
 }
@@ -112,8 +113,10 @@ int simk_context_destroy(simk_context* ctx) {
         cudaSetDevice(ctx->impl.device);
         cudaStreamSynchronize(ctx->impl.stream);
         cudaStream_t s = ctx->impl.own_stream;
+        const int device = ctx->impl.device;
         delete ctx;
         if (s) cudaStreamDestroy(s);
+        device_context_gone(device);
     });
 }
 
@@ -353,14 +356,7 @@ int simk_potential_read_transmission(simk_context* ctx, simk_potential* potentia
         activate(ctx->impl);
         prepare_transmissions(ctx->impl, potential->impl, energy);
         const long long N = potential->impl.g.count();
-        std::vector<float2> h(N);
-        SIMK_CUDA(cudaStreamSynchronize(ctx->impl.stream));  // the copy below is not ordered after that stream
-        SIMK_CUDA(cudaMemcpy(h.data(), potential->impl.t.as<float2>() + slice * N, N * sizeof(float2),
-                             cudaMemcpyDeviceToHost));
-        for (long long i = 0; i < N; ++i) {
-            re[i] = h[i].x;
-            im[i] = h[i].y;
-        }
+        download_complex(ctx->impl, potential->impl.t.as<float2>() + slice * N, N, re, im);
     });
 }
 
@@ -578,13 +574,7 @@ int simk_build_probes(simk_context* ctx, const simk_grid* grid, const simk_probe
         launch_probes(c, g, spectrum.as<float2>(), rx.as<float2>(), ry.as<float2>(), count, psi.as<float2>(), 1.0f);
         fft2(c.plan(g.ny, 32), c.plan(g.nx, 32), psi.ptr, g.nx, g.ny, count, +1, 1.0 / (double)N, c.stream,
              &c.launches);
-        std::vector<float2> h(count * N);
-        SIMK_CUDA(cudaMemcpyAsync(h.data(), psi.ptr, count * N * sizeof(float2), cudaMemcpyDeviceToHost, c.stream));
-        SIMK_CUDA(cudaStreamSynchronize(c.stream));
-        for (long long i = 0; i < count * N; ++i) {
-            out_re[i] = h[i].x;
-            out_im[i] = h[i].y;
-        }
+        download_complex(c, psi.as<float2>(), count * N, out_re, out_im);
     });
 }
 

@@ -60,27 +60,33 @@ template <typename V, typename S> __host__ __device__ __forceinline__ V mul_si(V
 template <typename V> __host__ __device__ __forceinline__ decltype(V::x) cabs2(V a) { return a.x * a.x + a.y * a.y; }
 
 // ---- device buffers -------------------------------------------------------------------------------------------------
+// Blocks come from and go back to the ones kept per device (hostio.cu).
+void* device_alloc(size_t n, size_t* got, int* device);
+void device_free(void* p, size_t bytes, int device);
+void device_context_made(int device);
+void device_context_gone(int device);
+
 struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
+    int device = 0;
     DeviceBuffer() = default;
     explicit DeviceBuffer(size_t n) { alloc(n); }
     DeviceBuffer(const DeviceBuffer&) = delete;
     DeviceBuffer& operator=(const DeviceBuffer&) = delete;
-    DeviceBuffer(DeviceBuffer&& o) noexcept : ptr(o.ptr), bytes(o.bytes) { o.ptr = nullptr; o.bytes = 0; }
+    DeviceBuffer(DeviceBuffer&& o) noexcept : ptr(o.ptr), bytes(o.bytes), device(o.device) { o.ptr = nullptr; o.bytes = 0; }
     DeviceBuffer& operator=(DeviceBuffer&& o) noexcept {
-        if (this != &o) { release(); ptr = o.ptr; bytes = o.bytes; o.ptr = nullptr; o.bytes = 0; }
+        if (this != &o) { release(); ptr = o.ptr; bytes = o.bytes; device = o.device; o.ptr = nullptr; o.bytes = 0; }
         return *this;
     }
     ~DeviceBuffer() { release(); }
     void alloc(size_t n) {
         release();
         if (n == 0) return;
-        SIMK_CUDA(cudaMalloc(&ptr, n));
-        bytes = n;
+        ptr = device_alloc(n, &bytes, &device);
     }
     void ensure(size_t n) { if (bytes < n) alloc(n); }
-    void release() { if (ptr) { cudaFree(ptr); ptr = nullptr; bytes = 0; } }
+    void release() { if (ptr) { device_free(ptr, bytes, device); ptr = nullptr; bytes = 0; } }
     template <typename T> T* as() const { return static_cast<T*>(ptr); }
 };
 

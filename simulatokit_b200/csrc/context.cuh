@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "fft.cuh"
+#include "hostio.cuh"
 
 struct simk_context;
 struct simk_potential;
@@ -179,6 +180,7 @@ struct Context {
     const int* wave_p = nullptr;
     int wave_p_blocks = 0;
     std::map<std::pair<int, int>, std::unique_ptr<LinePlan>> plans;
+    HostStage stage;  // pinned halves between split float64 host arrays and complex64 device arrays
     DeviceBuffer lobato_elements;  // the scaled Lobato parameters of Z = 1 .. 103
     DeviceBuffer evaluate_work;    // the surrogate's queries, their full projections and results
     std::map<int, DeviceBuffer> twopass_tables;  // the two-pass engine's twiddles by line length

@@ -72,15 +72,11 @@ void run_waves(Context& ctx, PotentialImpl& pot, double energy, double tx, doubl
     prepare_transmissions(ctx, pot, energy);
     const long long B = batch_size(ctx, g, count);
     ctx.work_a.ensure(B * N * sizeof(float2));
-    std::vector<float2> host(B * N);
     const int np = (int)planes.size();
     for (long long first = 0; first < count; first += B) {
         const int b = (int)std::min<long long>(B, count - first);
-        for (long long i = 0; i < b * N; ++i)
-            host[i] = make_float2((float)in_re[first * N + i], (float)in_im[first * N + i]);
-        SIMK_CUDA(cudaMemcpyAsync(ctx.work_a.ptr, host.data(), b * N * sizeof(float2), cudaMemcpyHostToDevice,
-                                  ctx.stream));
         float2* psi = ctx.work_a.as<float2>();
+        upload_complex(ctx, psi, in_re + first * N, in_im + first * N, b * N);
         const bool fused = (ctx.form != SIMK_FORM_PLAIN) && fused_supported(ctx, g);
         if (fused) ctx.work_b.ensure(B * N * sizeof(float2));
         auto copy_out = [&](int j) {
@@ -93,15 +89,15 @@ void run_waves(Context& ctx, PotentialImpl& pot, double energy, double tx, doubl
                     finish_rows(ctx, g, ctx.work_b.as<float2>(), b);
                     src = ctx.work_b.as<float2>();
                 }
-                SIMK_CUDA(cudaMemcpyAsync(host.data(), src, b * N * sizeof(float2), cudaMemcpyDeviceToHost, ctx.stream));
-                SIMK_CUDA(cudaStreamSynchronize(ctx.stream));
                 // output layout: [wave][plane][N] for run (count = 1) and [wave][N] for run_batch (one plane)
-                for (int w = 0; w < b; ++w)
-                    for (long long i = 0; i < N; ++i) {
-                        const long long o = ((first + w) * np + q) * N + i;
-                        out_re[o] = host[w * N + i].x;
-                        out_im[o] = host[w * N + i].y;
+                if (np == 1) {
+                    download_complex(ctx, src, b * N, out_re + first * N, out_im + first * N);
+                } else {
+                    for (int w = 0; w < b; ++w) {
+                        const long long o = ((first + w) * np + q) * N;
+                        download_complex(ctx, src + w * N, N, out_re + o, out_im + o);
                     }
+                }
             }
         };
         if (fused)
@@ -285,7 +281,6 @@ void scan_waves(Context& ctx, const simk_probe& probe, PotentialImpl& pot, int n
     const bool fused = (ctx.form != SIMK_FORM_PLAIN) && fused_supported(ctx, g);
     if (fused) ctx.work_b.ensure(B * N * sizeof(float2));
     DeviceBuffer outb((size_t)B * M * sizeof(float2));
-    std::vector<float2> h((size_t)B * M);
     const LinePlan& prow = ctx.plan(g.ny, 32);
     const LinePlan& pcol = ctx.plan(g.nx, 32);
     for (long long first = 0; first < n_pos; first += B) {
@@ -310,13 +305,7 @@ void scan_waves(Context& ctx, const simk_probe& probe, PotentialImpl& pot, int n
         ++ctx.launches;
         fft2(ctx.plan(columns, 32), ctx.plan(rows, 32), outb.ptr, rows, columns, b, +1, 1.0, ctx.stream,
              &ctx.launches);
-        SIMK_CUDA(cudaMemcpyAsync(h.data(), outb.ptr, (size_t)total * sizeof(float2), cudaMemcpyDeviceToHost,
-                                  ctx.stream));
-        SIMK_CUDA(cudaStreamSynchronize(ctx.stream));
-        for (long long i = 0; i < total; ++i) {
-            out_re[first * M + i] = h[i].x;
-            out_im[first * M + i] = h[i].y;
-        }
+        download_complex(ctx, outb.as<float2>(), total, out_re + first * M, out_im + first * M);
     }
     check_device_error(ctx);
 }

@@ -188,9 +188,11 @@ void build_potential_from_atoms(Context& ctx, PotentialImpl& pot, int pi_choice,
     std::vector<int> pix;
     std::vector<double> wts;
     std::vector<long long> group_ptr(1, 0);
-    std::vector<double> dense(N, 0.0);
-    std::vector<char> touched(N, 0);
-    std::vector<int> touched_list;
+    struct Weight {
+        int pixel, order;
+        double w;
+    };
+    std::vector<Weight> entries;
     std::vector<std::vector<int>> atoms_of(S * E);
     for (int a = 0; a < n_atoms; ++a) {
         int e = (int)(std::lower_bound(elements.begin(), elements.end(), Z[a]) - elements.begin());
@@ -200,7 +202,7 @@ void build_potential_from_atoms(Context& ctx, PotentialImpl& pot, int pi_choice,
     for (int j = 0; j < S; ++j) {
         for (int e = 0; e < E; ++e) {
             const auto& list = atoms_of[j * E + e];
-            touched_list.clear();
+            entries.clear();
             for (int k = 0; k < 4; ++k) {
                 for (int a : list) {
                     const double px = xyz[3 * a] / g.dx(), py = xyz[3 * a + 1] / g.dy();
@@ -210,19 +212,19 @@ void build_potential_from_atoms(Context& ctx, PotentialImpl& pot, int pi_choice,
                     const long long i = mod((long long)r + ((k == 1 || k == 3) ? 1 : 0), g.nx);
                     const long long jj = mod((long long)c + ((k >= 2) ? 1 : 0), g.ny);
                     const long long p = i * g.ny + jj;
-                    if (!touched[p]) {
-                        touched[p] = 1;
-                        touched_list.push_back((int)p);
-                    }
-                    dense[p] += w;
+                    entries.push_back({(int)p, (int)entries.size(), w});
                 }
             }
-            std::sort(touched_list.begin(), touched_list.end());
-            for (int p : touched_list) {
+            // by pixel, a pixel's weights in their order: the same sums as into a dense image, without one
+            std::sort(entries.begin(), entries.end(), [](const Weight& a, const Weight& b) {
+                return a.pixel != b.pixel ? a.pixel < b.pixel : a.order < b.order;
+            });
+            for (size_t i = 0; i < entries.size();) {
+                double sum = 0.0;
+                const int p = entries[i].pixel;
+                for (; i < entries.size() && entries[i].pixel == p; ++i) sum += entries[i].w;
                 pix.push_back(p);
-                wts.push_back(dense[p]);
-                dense[p] = 0.0;
-                touched[p] = 0;
+                wts.push_back(sum);
             }
             group_ptr.push_back((long long)pix.size());
         }
@@ -529,27 +531,16 @@ void apply_ctf_device(Context& ctx, const GridGeom& g, double energy, const simk
     SIMK_CUDA(cudaGetLastError());
     const long long B = std::max<long long>(1, std::min<long long>(count, (256LL << 20) / (N * (long long)sizeof(float2))));
     DeviceBuffer psi(B * N * sizeof(float2));
-    std::vector<float2> h(B * N);
     const LinePlan& prow = ctx.plan(g.ny, 32);
     const LinePlan& pcol = ctx.plan(g.nx, 32);
     for (long long first = 0; first < count; first += B) {
         const int b = (int)std::min<long long>(B, count - first);
-        for (long long i = 0; i < b * N; ++i)
-            h[i] = make_float2((float)in_re[first * N + i], (float)in_im[first * N + i]);
-        SIMK_CUDA(cudaMemcpyAsync(psi.ptr, h.data(), b * N * sizeof(float2), cudaMemcpyHostToDevice, ctx.stream));
+        upload_complex(ctx, psi.as<float2>(), in_re + first * N, in_im + first * N, b * N);
         fft2(prow, pcol, psi.ptr, g.nx, g.ny, b, -1, 1.0, ctx.stream, &ctx.launches);
         launch_mul_broadcast(ctx, psi.as<float2>(), h32.as<float2>(), N, b, 1.0f / (float)N);
         fft2(prow, pcol, psi.ptr, g.nx, g.ny, b, +1, 1.0, ctx.stream, &ctx.launches);
-        SIMK_CUDA(cudaMemcpyAsync(h.data(), psi.ptr, b * N * sizeof(float2), cudaMemcpyDeviceToHost, ctx.stream));
-        SIMK_CUDA(cudaStreamSynchronize(ctx.stream));
-        for (long long i = 0; i < b * N; ++i) {
-            const double re = h[i].x, im = h[i].y;
-            if (out_re) {
-                out_re[first * N + i] = re;
-                out_im[first * N + i] = im;
-            }
-            if (out_intensity) out_intensity[first * N + i] = re * re + im * im;
-        }
+        download_complex(ctx, psi.as<float2>(), b * N, out_re ? out_re + first * N : nullptr,
+                         out_im ? out_im + first * N : nullptr, out_intensity ? out_intensity + first * N : nullptr);
     }
 }
 

@@ -15,7 +15,7 @@ import numpy as np
 from . import _lib as L
 from .core import Grid, Waves, _refuse
 from .engine import Engine, ExecutionOptions
-from .multislice import Backend
+from .multislice import Backend, _join
 
 
 class AnnularDetector:
@@ -149,7 +149,7 @@ def _waves_scan(probe, potential, scan, detector: WavesDetector, engine: Engine)
     L.check(engine.lib.simk_scan_waves(engine.handle, C.byref(p), h, n, L.dptr(positions), detector.rows or 0,
                                        detector.columns or 0, L.dptr(re), L.dptr(im)))
     grid = Grid(rows, columns, probe.grid.extent_x, probe.grid.extent_y)
-    return ScanWaves(list(scan.shape), grid, probe.beam, (re + 1j * im).reshape(n, rows, columns))
+    return ScanWaves(list(scan.shape), grid, probe.beam, _join(re, im).reshape(n, rows, columns))
 
 
 def _check_waves_memory(probe, scan, detector: WavesDetector, configurations: int, limit: int | None):

@@ -433,6 +433,12 @@ def _split(field: np.ndarray):
     return np.ascontiguousarray(a.real), np.ascontiguousarray(a.imag)
 
 
+def _join(re: np.ndarray, im: np.ndarray) -> np.ndarray:
+    out = np.empty(re.shape, dtype=np.complex128)
+    out.real, out.imag = re, im
+    return out
+
+
 class Multislice:
     """Multislice.run / runBatch / transmissionFunctions on the CUDA backend."""
 
@@ -456,7 +462,7 @@ class Multislice:
                                float(incident.tilt[1]), L.dptr(re), L.dptr(im), len(dev_planes), L.iptr(dev_planes),
                                L.dptr(ore), L.dptr(oim)))
         for q in range(len(dev_planes)):
-            out.append(Waves(ore[q] + 1j * oim[q], incident.grid, incident.beam, incident.normalization,
+            out.append(Waves(_join(ore[q], oim[q]), incident.grid, incident.beam, incident.normalization,
                              incident.tilt))
         return out
 
@@ -483,7 +489,7 @@ class Multislice:
         h = through.handle(e)
         L.check(e.lib.simk_run_batch(e.handle, h.handle, first.beam.energy, float(first.tilt[0]), float(first.tilt[1]),
                                      len(incidents), L.dptr(re), L.dptr(im), L.dptr(ore), L.dptr(oim)))
-        return [Waves(ore[k] + 1j * oim[k], w.grid, w.beam, w.normalization, w.tilt) for k, w in enumerate(incidents)]
+        return [Waves(_join(ore[k], oim[k]), w.grid, w.beam, w.normalization, w.tilt) for k, w in enumerate(incidents)]
 
     run_batch = runBatch
 

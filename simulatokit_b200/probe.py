@@ -182,8 +182,10 @@ class ContrastTransferFunction:
         g, c = grid.c(), self.c()
         L.check(e.lib.simk_apply_ctf(e.handle, C.byref(g), float(beam.energy), C.byref(c), len(ws), L.dptr(re_in),
                                      L.dptr(im_in), L.dptr(re), L.dptr(im), L.dptr(inten)))
-        out = [Waves((re[k * n:(k + 1) * n] + 1j * im[k * n:(k + 1) * n]).reshape(grid.nx, grid.ny), grid, w.beam,
-                     w.normalization) for k, w in enumerate(ws)]
+        field = np.empty(len(ws) * n, dtype=np.complex128)
+        field.real, field.imag = re, im
+        out = [Waves(field[k * n:(k + 1) * n].reshape(grid.nx, grid.ny), grid, w.beam, w.normalization)
+               for k, w in enumerate(ws)]
         images = [inten[k * n:(k + 1) * n].reshape(grid.nx, grid.ny) for k in range(len(ws))]
         return (out, images) if many else (out[0], images[0])
 

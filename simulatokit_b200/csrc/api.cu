@@ -275,7 +275,7 @@ int simk_potential_from_values(simk_context* ctx, const simk_grid* grid, int32_t
         p->impl.dz = checked_thickness(n_slices, thickness);
         const size_t bytes = (size_t)n_slices * p->impl.g.count() * sizeof(double);
         p->impl.V.alloc(bytes);
-        SIMK_CUDA(cudaMemcpy(p->impl.V.ptr, values, bytes, cudaMemcpyHostToDevice));
+        copy_to_device(p->impl.V.ptr, values, bytes);
         *out = p.release();
     });
 }
@@ -715,7 +715,7 @@ int simk_fft2(simk_context* ctx, int32_t nx, int32_t ny, int32_t count, int32_t 
             std::vector<double2> h(total);
             for (long long i = 0; i < total; ++i) h[i] = make_double2(in_re[i], in_im[i]);
             DeviceBuffer d(total * sizeof(double2));
-            SIMK_CUDA(cudaMemcpy(d.ptr, h.data(), total * sizeof(double2), cudaMemcpyHostToDevice));
+            copy_to_device(d.ptr, h.data(), total * sizeof(double2));
             fft2(c.plan(ny, 64), c.plan(nx, 64), d.ptr, nx, ny, count, inverse ? +1 : -1, scale, c.stream, &c.launches);
             SIMK_CUDA(cudaStreamSynchronize(c.stream));
             SIMK_CUDA(cudaMemcpy(h.data(), d.ptr, total * sizeof(double2), cudaMemcpyDeviceToHost));
@@ -727,7 +727,7 @@ int simk_fft2(simk_context* ctx, int32_t nx, int32_t ny, int32_t count, int32_t 
             std::vector<float2> h(total);
             for (long long i = 0; i < total; ++i) h[i] = make_float2((float)in_re[i], (float)in_im[i]);
             DeviceBuffer d(total * sizeof(float2));
-            SIMK_CUDA(cudaMemcpy(d.ptr, h.data(), total * sizeof(float2), cudaMemcpyHostToDevice));
+            copy_to_device(d.ptr, h.data(), total * sizeof(float2));
             fft2(c.plan(ny, 32), c.plan(nx, 32), d.ptr, nx, ny, count, inverse ? +1 : -1, scale, c.stream, &c.launches);
             SIMK_CUDA(cudaStreamSynchronize(c.stream));
             SIMK_CUDA(cudaMemcpy(h.data(), d.ptr, total * sizeof(float2), cudaMemcpyDeviceToHost));
@@ -858,7 +858,7 @@ int simk_surrogate_parameters(simk_context* ctx, simk_surrogate* surrogate, floa
         }
         if (set) {
             SIMK_CUDA(cudaStreamSynchronize(ctx->impl.stream));  // no launch in flight still reads the old values
-            SIMK_CUDA(cudaMemcpy(s.params.ptr, set, kSurrogateParams * sizeof(float), cudaMemcpyHostToDevice));
+            copy_to_device(s.params.ptr, set, kSurrogateParams * sizeof(float));
             if (ms && !get) {
                 s.y_mean = ms[0];
                 s.y_std = ms[1];

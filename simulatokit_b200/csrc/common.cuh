@@ -33,6 +33,13 @@ inline void check_cuda(cudaError_t e, const char* what) {
 #define SIMK_REQUIRE(cond, msg) \
     do { if (!(cond)) throw ::simk::Error(SIMK_ERR_INVALID, (msg)); } while (0)
 
+// A host array to the device, there when this returns: a plain cudaMemcpy from pageable memory may return while its last
+// part is still on the way, which a kernel on a non-blocking stream (every context's) would not wait for.
+inline void copy_to_device(void* dst, const void* src, size_t bytes) {
+    SIMK_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+    SIMK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+}
+
 // ---- complex arithmetic on float2 / double2 -------------------------------------------------------------------------
 template <typename T> struct C2;
 template <> struct C2<float> { using type = float2; };

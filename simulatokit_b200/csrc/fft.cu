@@ -77,7 +77,7 @@ void upload_complex(DeviceBuffer& buf, const std::vector<std::complex<double>>& 
         h[i].y = (decltype(V::x))v[i].imag();
     }
     buf.alloc(h.size() * sizeof(V));
-    SIMK_CUDA(cudaMemcpy(buf.ptr, h.data(), h.size() * sizeof(V), cudaMemcpyHostToDevice));
+    copy_to_device(buf.ptr, h.data(), h.size() * sizeof(V));
 }
 
 std::vector<std::complex<double>> twiddles(int m) {
@@ -150,8 +150,8 @@ std::unique_ptr<LinePlan> make_line_plan(int n, int precision) {
     }
     p->rad_cos.alloc(rc.size() * sizeof(double));
     p->rad_sin.alloc(rs.size() * sizeof(double));
-    SIMK_CUDA(cudaMemcpy(p->rad_cos.ptr, rc.data(), rc.size() * sizeof(double), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(p->rad_sin.ptr, rs.data(), rs.size() * sizeof(double), cudaMemcpyHostToDevice));
+    copy_to_device(p->rad_cos.ptr, rc.data(), rc.size() * sizeof(double));
+    copy_to_device(p->rad_sin.ptr, rs.data(), rs.size() * sizeof(double));
     return p;
 }
 

@@ -291,7 +291,7 @@ void infinite_points(Context& ctx, int n, const int* z_dev, const double* rho_de
         std::vector<ElementAB> ab;
         for (int z = 1; z <= 103; ++z) ab.push_back(element_ab(z));
         DeviceBuffer made(ab.size() * sizeof(ElementAB));
-        SIMK_CUDA(cudaMemcpy(made.ptr, ab.data(), ab.size() * sizeof(ElementAB), cudaMemcpyHostToDevice));
+        copy_to_device(made.ptr, ab.data(), ab.size() * sizeof(ElementAB));
         ctx.lobato_elements = std::move(made);
     }
     k_infinite_points<<<(n + 127) / 128, 128, 0, ctx.stream>>>(z_dev, rho_dev, n, ctx.lobato_elements.as<ElementAB>(),
@@ -329,11 +329,11 @@ FiniteDevice upload_finite(Context& ctx, const FiniteSetup& s, DeviceBuffer& pai
     rmin.alloc(std::max<size_t>(1, s.rmin.size()) * sizeof(double));
     rcut.alloc(std::max<size_t>(1, s.rcut.size()) * sizeof(double));
     if (!s.pairs.empty())
-        SIMK_CUDA(cudaMemcpy(pairs.ptr, s.pairs.data(), s.pairs.size() * sizeof(FinitePair), cudaMemcpyHostToDevice));
+        copy_to_device(pairs.ptr, s.pairs.data(), s.pairs.size() * sizeof(FinitePair));
     if (!s.ab.empty()) {
-        SIMK_CUDA(cudaMemcpy(ab.ptr, s.ab.data(), s.ab.size() * sizeof(ElementAB), cudaMemcpyHostToDevice));
-        SIMK_CUDA(cudaMemcpy(rmin.ptr, s.rmin.data(), s.rmin.size() * sizeof(double), cudaMemcpyHostToDevice));
-        SIMK_CUDA(cudaMemcpy(rcut.ptr, s.rcut.data(), s.rcut.size() * sizeof(double), cudaMemcpyHostToDevice));
+        copy_to_device(ab.ptr, s.ab.data(), s.ab.size() * sizeof(ElementAB));
+        copy_to_device(rmin.ptr, s.rmin.data(), s.rmin.size() * sizeof(double));
+        copy_to_device(rcut.ptr, s.rcut.data(), s.rcut.size() * sizeof(double));
     }
     FiniteDevice d{};
     d.pairs = pairs.as<FinitePair>();
@@ -416,7 +416,7 @@ void build_potential_finite(Context& ctx, PotentialImpl& pot, int n_atoms, const
     auto run_quadrature = [&](const std::vector<int>& ids) {
         if (ids.empty()) return;
         DeviceBuffer did(ids.size() * sizeof(int));
-        SIMK_CUDA(cudaMemcpy(did.ptr, ids.data(), ids.size() * sizeof(int), cudaMemcpyHostToDevice));
+        copy_to_device(did.ptr, ids.data(), ids.size() * sizeof(int));
         KernelTimer t(ctx, "finite_quadrature", 0.0);
         k_finite_profiles_ids<<<blocks_for((long long)ids.size() * nr), 256, 0, ctx.stream>>>(
             d.pairs, did.as<int>(), (int)ids.size(), d.ab, d.rmin, d.rcut, nr, table.as<double>());
@@ -440,10 +440,10 @@ void build_potential_finite(Context& ctx, PotentialImpl& pot, int n_atoms, const
             }
         const std::vector<double> pinf = infinite_profiles(ctx, tz, trho);
         DeviceBuffer drf(rf.size() * sizeof(float2));
-        SIMK_CUDA(cudaMemcpy(drf.ptr, rf.data(), rf.size() * sizeof(float2), cudaMemcpyHostToDevice));
-        SIMK_CUDA(cudaMemcpy(did.ptr, in_dom.data(), in_dom.size() * sizeof(int), cudaMemcpyHostToDevice));
-        SIMK_CUDA(cudaMemcpy(dz.ptr, s.elements.data(), s.elements.size() * sizeof(int), cudaMemcpyHostToDevice));
-        SIMK_CUDA(cudaMemcpy(dpinf.ptr, pinf.data(), pinf.size() * sizeof(double), cudaMemcpyHostToDevice));
+        copy_to_device(drf.ptr, rf.data(), rf.size() * sizeof(float2));
+        copy_to_device(did.ptr, in_dom.data(), in_dom.size() * sizeof(int));
+        copy_to_device(dz.ptr, s.elements.data(), s.elements.size() * sizeof(int));
+        copy_to_device(dpinf.ptr, pinf.data(), pinf.size() * sizeof(double));
         surrogate_profiles(ctx, *sg, d, did.as<int>(), (int)in_dom.size(), dz.as<int>(), drf.as<float2>(),
                            dpinf.as<double>(), nr, table.as<double>());
         SIMK_CUDA(cudaStreamSynchronize(ctx.stream));

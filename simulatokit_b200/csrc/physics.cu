@@ -871,12 +871,12 @@ std::unique_ptr<DetectorPlan> build_detector_plan(Context& ctx, const GridGeom& 
                     ptr.push_back((int)idx.size());
                 }
                 P.alloc(ptr.size() * sizeof(int));
-                SIMK_CUDA(cudaMemcpy(P.ptr, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+                copy_to_device(P.ptr, ptr.data(), ptr.size() * sizeof(int));
                 I.alloc(std::max<size_t>(1, idx.size()) * sizeof(int));
                 W.alloc(std::max<size_t>(1, wt.size()) * sizeof(double));
                 if (!idx.empty()) {
-                    SIMK_CUDA(cudaMemcpy(I.ptr, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice));
-                    SIMK_CUDA(cudaMemcpy(W.ptr, wt.data(), wt.size() * sizeof(double), cudaMemcpyHostToDevice));
+                    copy_to_device(I.ptr, idx.data(), idx.size() * sizeof(int));
+                    copy_to_device(W.ptr, wt.data(), wt.size() * sizeof(double));
                 }
             };
             axis(g.nx, a.ax, d.nr, b->xp, b->xi, b->xw);
@@ -906,16 +906,16 @@ std::unique_ptr<DetectorPlan> build_detector_plan(Context& ctx, const GridGeom& 
     plan->total_entries = (long long)pix.size();
     plan->total_crop = (long long)crop.size();
     plan->chan_ptr.alloc(ptr.size() * sizeof(int));
-    SIMK_CUDA(cudaMemcpy(plan->chan_ptr.ptr, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+    copy_to_device(plan->chan_ptr.ptr, ptr.data(), ptr.size() * sizeof(int));
     if (!pix.empty()) {
         plan->chan_pix.alloc(pix.size() * sizeof(int));
         plan->chan_w.alloc(w.size() * sizeof(float));
-        SIMK_CUDA(cudaMemcpy(plan->chan_pix.ptr, pix.data(), pix.size() * sizeof(int), cudaMemcpyHostToDevice));
-        SIMK_CUDA(cudaMemcpy(plan->chan_w.ptr, w.data(), w.size() * sizeof(float), cudaMemcpyHostToDevice));
+        copy_to_device(plan->chan_pix.ptr, pix.data(), pix.size() * sizeof(int));
+        copy_to_device(plan->chan_w.ptr, w.data(), w.size() * sizeof(float));
     }
     if (!crop.empty()) {
         plan->crop_src.alloc(crop.size() * sizeof(int));
-        SIMK_CUDA(cudaMemcpy(plan->crop_src.ptr, crop.data(), crop.size() * sizeof(int), cudaMemcpyHostToDevice));
+        copy_to_device(plan->crop_src.ptr, crop.data(), crop.size() * sizeof(int));
     }
     return plan;
 }
@@ -949,10 +949,10 @@ const DetectorPlan::TileChannels& DetectorPlan::tiles(int tc) {
         ptr.push_back((int)ent.size());
     }
     t->ptr.alloc(ptr.size() * sizeof(int));
-    SIMK_CUDA(cudaMemcpy(t->ptr.ptr, ptr.data(), ptr.size() * sizeof(int), cudaMemcpyHostToDevice));
+    copy_to_device(t->ptr.ptr, ptr.data(), ptr.size() * sizeof(int));
     t->ent.alloc(std::max<size_t>(1, ent.size()) * sizeof(int2));
     if (!ent.empty())
-        SIMK_CUDA(cudaMemcpy(t->ent.ptr, ent.data(), ent.size() * sizeof(int2), cudaMemcpyHostToDevice));
+        copy_to_device(t->ent.ptr, ent.data(), ent.size() * sizeof(int2));
     tile_channels.push_back(std::move(t));
     return *tile_channels.back();
 }

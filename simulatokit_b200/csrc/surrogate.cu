@@ -655,11 +655,11 @@ void surrogate_quadrature_points(Context& ctx, const std::vector<int>& z, const 
     for (int i = 0; i < n; ++i) idx[i] = (int)(std::lower_bound(els.begin(), els.end(), z[i]) - els.begin());
     DeviceBuffer dab(ab.size() * sizeof(ElementAB)), didx(n * sizeof(int)), dr(n * sizeof(double)),
         dl(n * sizeof(double)), du(n * sizeof(double));
-    SIMK_CUDA(cudaMemcpy(dab.ptr, ab.data(), ab.size() * sizeof(ElementAB), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(didx.ptr, idx.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(dr.ptr, rho.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(dl.ptr, zl.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(du.ptr, zu.data(), n * sizeof(double), cudaMemcpyHostToDevice));
+    copy_to_device(dab.ptr, ab.data(), ab.size() * sizeof(ElementAB));
+    copy_to_device(didx.ptr, idx.data(), n * sizeof(int));
+    copy_to_device(dr.ptr, rho.data(), n * sizeof(double));
+    copy_to_device(dl.ptr, zl.data(), n * sizeof(double));
+    copy_to_device(du.ptr, zu.data(), n * sizeof(double));
     finite_points(ctx, dab.as<ElementAB>(), n, didx.as<int>(), dr.as<double>(), dl.as<double>(), du.as<double>(),
                   out_dev);
     SIMK_CUDA(cudaStreamSynchronize(ctx.stream));
@@ -697,7 +697,7 @@ std::unique_ptr<SurrogateImpl> surrogate_train(Context& ctx, const std::vector<i
     fill(OFF_W2, kHidden * kHidden, kHidden);
     fill(OFF_W3, kHidden * kHidden, kHidden);
     fill(OFF_W4, kHidden, kHidden);
-    SIMK_CUDA(cudaMemcpy(s->params.ptr, p.data(), kSurrogateParams * sizeof(float), cudaMemcpyHostToDevice));
+    copy_to_device(s->params.ptr, p.data(), kSurrogateParams * sizeof(float));
     SIMK_CUDA(cudaMemset(s->m.ptr, 0, kSurrogateParams * sizeof(float)));
     SIMK_CUDA(cudaMemset(s->v.ptr, 0, kSurrogateParams * sizeof(float)));
     // the training set, labelled F = P / P_inf with P by the float64 device quadrature
@@ -733,14 +733,12 @@ std::unique_ptr<SurrogateImpl> surrogate_train(Context& ctx, const std::vector<i
         std::vector<float> rf;
         for (long long k = 0; k < nb; ++k) {
             fill_rows(all_z, all_rho, all_zl, all_zu, (size_t)k * batch, batch, rz, rf);
-            SIMK_CUDA(cudaMemcpy(rows_z.as<int>() + k * 2 * batch, rz.data(), rz.size() * sizeof(int),
-                                 cudaMemcpyHostToDevice));
-            SIMK_CUDA(cudaMemcpy(rows_f.as<float>() + k * 4 * batch, rf.data(), rf.size() * sizeof(float),
-                                 cudaMemcpyHostToDevice));
+            copy_to_device(rows_z.as<int>() + k * 2 * batch, rz.data(), rz.size() * sizeof(int));
+            copy_to_device(rows_f.as<float>() + k * 4 * batch, rf.data(), rf.size() * sizeof(float));
         }
     }
     DeviceBuffer targets((size_t)n * sizeof(float));
-    SIMK_CUDA(cudaMemcpy(targets.ptr, all_F.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+    copy_to_device(targets.ptr, all_F.data(), n * sizeof(float));
     Batch b;
     b.ensure(batch);
     const float b1 = 0.9f, b2 = 0.999f;
@@ -830,9 +828,9 @@ double surrogate_gradients(Context& ctx, SurrogateImpl& s, const std::vector<int
     std::vector<float> rf, y(B);
     fill_rows(z, rho, zl, zu, 0, B, rz, rf);
     for (int i = 0; i < B; ++i) y[i] = (float)target[i];
-    SIMK_CUDA(cudaMemcpy(b.z.ptr, rz.data(), rz.size() * sizeof(int), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(b.feats.ptr, rf.data(), rf.size() * sizeof(float), cudaMemcpyHostToDevice));
-    SIMK_CUDA(cudaMemcpy(b.target.ptr, y.data(), B * sizeof(float), cudaMemcpyHostToDevice));
+    copy_to_device(b.z.ptr, rz.data(), rz.size() * sizeof(int));
+    copy_to_device(b.feats.ptr, rf.data(), rf.size() * sizeof(float));
+    copy_to_device(b.target.ptr, y.data(), B * sizeof(float));
     const double loss = forward_backward(ctx, s.params.as<float>(), s.grads.as<float>(), b.z.as<int>(),
                                          b.feats.as<float>(), b.target.as<float>(), B, b, true);
     SIMK_CUDA(cudaMemcpy(grads_host, s.grads.ptr, kSurrogateParams * sizeof(float), cudaMemcpyDeviceToHost));

@@ -44,7 +44,7 @@ const float2* twopass_table(Context& ctx, int n) {
             h[i] = make_float2((float)w.c, (float)w.s);
         }
         DeviceBuffer made(n * sizeof(float2));
-        SIMK_CUDA(cudaMemcpy(made.ptr, h.data(), n * sizeof(float2), cudaMemcpyHostToDevice));
+        copy_to_device(made.ptr, h.data(), n * sizeof(float2));
         buf = std::move(made);
     }
     return buf.as<float2>();

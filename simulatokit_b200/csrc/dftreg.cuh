@@ -1,4 +1,4 @@
-// dftreg.cuh -- DFTs of a compile-time length held in one thread's registers (float2, natural order in and out):
+// dftreg.cuh -- DFTs of a compile-time length held in one thread's registers (float2 or double2, natural order in and out):
 // 2, 3, 4, 5 and 8 directly, the other lengths as A x B Cooley-Tukey steps whose twiddles are constants of the
 // unrolled code. DIR = -1 forward (e^{-2 pi i jk/R}), +1 inverse, unnormalised.
 #pragma once
@@ -140,6 +140,27 @@ template <int DIR> __device__ __forceinline__ void pbfly8(float2 (&v)[8]) {
     v[7] = psub(e[3], o3);
 }
 
+// The same in float64, with constants rounded to nearest.
+template <int E, int N, int DIR> __device__ __forceinline__ double2 wmul(double2 v) {
+    constexpr int e = ((E % N) + N) % N;
+    constexpr double h = 0.70710678118654752440;
+    if constexpr (e == 0) return v;
+    else if constexpr (2 * e == N) return make_double2(-v.x, -v.y);
+    else if constexpr (4 * e == N) return make_double2(-DIR * v.y, DIR * v.x);
+    else if constexpr (4 * e == 3 * N) return make_double2(DIR * v.y, -DIR * v.x);
+    else if constexpr (8 * e == N) return make_double2((v.x - DIR * v.y) * h, (v.y + DIR * v.x) * h);
+    else if constexpr (8 * e == 3 * N) return make_double2((-v.x - DIR * v.y) * h, (-v.y + DIR * v.x) * h);
+    else if constexpr (8 * e == 5 * N) return make_double2((DIR * v.y - v.x) * h, (-v.y - DIR * v.x) * h);
+    else if constexpr (8 * e == 7 * N) return make_double2((v.x + DIR * v.y) * h, (v.y - DIR * v.x) * h);
+    else {
+        constexpr double c = unit_cos(e, N), s = DIR * unit_sin(e, N);
+        return make_double2(v.x * c - v.y * s, v.y * c + v.x * s);
+    }
+}
+template <int DIR> __device__ __forceinline__ void pbfly3(double2 (&v)[3]) { bfly3<DIR>(v); }
+template <int DIR> __device__ __forceinline__ void pbfly5(double2 (&v)[5]) { bfly5<DIR>(v); }
+template <int DIR> __device__ __forceinline__ void pbfly8(double2 (&v)[8]) { bfly8<DIR>(v); }
+
 // The first factor A of the step R = A B.
 constexpr int dft_first(int r) {
     return r == 6 ? 2 : r == 10 ? 2 : r == 12 ? 3 : r == 15 ? 3 : r == 16 ? 4 : r == 18 ? 3 : r == 20 ? 4 : r == 24 ? 3
@@ -147,7 +168,7 @@ constexpr int dft_first(int r) {
 }
 
 // X[k1 + A k2] = sum_n2 W_R^{n2 k1} W_B^{n2 k2} sum_n1 x[B n1 + n2] W_A^{n1 k1}
-template <int R, int DIR> __device__ __forceinline__ void dft_reg(float2 (&v)[R]) {
+template <int R, int DIR, typename V> __device__ __forceinline__ void dft_reg(V (&v)[R]) {
     if constexpr (R == 1) return;
     else if constexpr (R == 2) bfly2<DIR>(v);
     else if constexpr (R == 3) pbfly3<DIR>(v);
@@ -157,10 +178,10 @@ template <int R, int DIR> __device__ __forceinline__ void dft_reg(float2 (&v)[R]
     else {
         constexpr int A = dft_first(R), B = R / A;
         static_assert(A > 1 && A * B == R, "a register DFT of this length is not defined");
-        float2 w[R];
+        V w[R];
         sfor<B>([&](auto n2c) {
             constexpr int n2 = decltype(n2c)::value;
-            float2 u[A];
+            V u[A];
             sfor<A>([&](auto n1c) { u[decltype(n1c)::value] = v[B * decltype(n1c)::value + n2]; });
             dft_reg<A, DIR>(u);
             sfor<A>([&](auto k1c) {
@@ -170,7 +191,7 @@ template <int R, int DIR> __device__ __forceinline__ void dft_reg(float2 (&v)[R]
         });
         sfor<A>([&](auto k1c) {
             constexpr int k1 = decltype(k1c)::value;
-            float2 u[B];
+            V u[B];
             sfor<B>([&](auto n2c) { u[decltype(n2c)::value] = w[k1 * B + decltype(n2c)::value]; });
             dft_reg<B, DIR>(u);
             sfor<B>([&](auto k2c) { v[k1 + A * decltype(k2c)::value] = u[decltype(k2c)::value]; });

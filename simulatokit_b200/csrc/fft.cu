@@ -4,6 +4,9 @@
 #include <algorithm>
 #include <complex>
 
+#include "dftreg.cuh"
+#include "linefft.cuh"
+
 namespace simk {
 
 LinePlanDev LinePlan::dev() const {
@@ -132,6 +135,19 @@ std::unique_ptr<LinePlan> make_line_plan(int n, int precision) {
     auto tw = twiddles(p->m);
     if (precision == 64) upload_complex<double2>(p->tw, tw);
     else upload_complex<float2>(p->tw, tw);
+    // the one-exchange transforms: the lengths with a plan, and Bluestein's work lengths with one
+    if (const int r1 = line_first_radix(p->m); r1 && (!p->bluestein || line_bluestein_length(p->m))) {
+        std::vector<std::complex<double>> t(p->m);
+        for (int i = 0; i < p->m; ++i) {
+            t[i] = tw[(long long)(i / r1) * (i % r1) % p->m];
+            if (precision != 64 && t[i].real() != 0.0 && t[i].imag() != 0.0) {  // on the unit circle as floats (dftreg.cuh)
+                const UnitPair w = unit_pair(t[i].real(), t[i].imag());
+                t[i] = {w.c, w.s};
+            }
+        }
+        if (precision == 64) upload_complex<double2>(p->table, t);
+        else upload_complex<float2>(p->table, t);
+    }
     // cos/sin tables of the generic radices
     std::vector<double> rc, rs;
     for (int r : p->factors) {
@@ -237,6 +253,27 @@ void launch_t(const LinePlan& plan, void* data, long long nlines, int lines_per_
               long long elem_stride, long long batch_stride, int dir, double scale, cudaStream_t stream,
               int64_t* launches) {
     using V = c2_t<T>;
+    // Whole rows or columns of fields, of a length with a plan: the one-exchange kernels. Plain-form float32 passes, us a
+    // launch against the Stockham kernel below: 256^2 x 64 waves 73 -> 15, 512^2 x 64 344 -> 55 (0.78 -> 4.9 TB/s), 500^2
+    // x 64 314 -> 54, 768^2 x 32 360 -> 60, 331^2 x 64 (Bluestein over 1024 points) 439 -> 108.
+    const bool rows = elem_stride == 1 && line_stride == plan.n && batch_stride == (long long)lines_per_batch * plan.n;
+    const bool columns = line_stride == 1 && elem_stride == lines_per_batch &&
+                         batch_stride == (long long)lines_per_batch * plan.n && nlines % lines_per_batch == 0;
+    if (plan.table.ptr && (rows || columns)) {
+        LineArgs<V> a{};
+        a.data = static_cast<V*>(data);
+        a.table = plan.table.as<V>();
+        a.chirp = plan.chirp.as<V>();
+        a.khat = plan.khat.as<V>();
+        a.lines = nlines;
+        a.n = plan.n;
+        a.ny = columns ? lines_per_batch : 0;
+        a.conj = dir > 0;
+        a.scale = (T)scale;
+        launch_line_any<V>(plan.m, plan.bluestein, a, columns, stream);
+        if (launches) ++*launches;
+        return;
+    }
     const int lds = plan.m + ((plan.m % 2 == 0) ? 1 : 0);
     const size_t budget = 96 * 1024;
     int L = (int)std::max<size_t>(1, std::min<size_t>(16, budget / (2 * (size_t)lds * sizeof(V))));

@@ -205,6 +205,7 @@ struct LinePlan {
     bool bluestein = false;
     std::vector<int> factors;
     DeviceBuffer tw, chirp, khat, rad_cos, rad_sin;
+    DeviceBuffer table;  // the one-exchange transforms' twiddles (linefft.cuh), empty where they do not take the length
     std::vector<int> rad_off;
     LinePlanDev dev() const;
 };

@@ -24,14 +24,15 @@ template <int N> struct LineLen { static constexpr int R1 = 0, R2 = 0; };
 template <int N, typename V> struct LinePlanCfg {
     static constexpr int R1 = LineLen<N>::R1, R2 = LineLen<N>::R2, LD = R1 | 1;
     // threads an SM: the registers R2 values need
-    static constexpr int MAXT = (sizeof(V) == 8 ? (R2 <= 16 ? 768 : 512) : (R2 <= 16 ? 384 : 256));
+    static constexpr int RM = R1 > R2 ? R1 : R2;
+    static constexpr int MAXT = (sizeof(V) == 8 ? (RM <= 16 ? 768 : 512) : (RM <= 16 ? 384 : 256));
     // rows: lines a block
     static constexpr int L = 128 / R2 > 0 ? 128 / R2 : 1;
     static constexpr int NT_ROWS = (L * R2 + 31) / 32 * 32;
     static constexpr int QB_ROWS = (L * R1 + NT_ROWS - 1) / NT_ROWS;
     // columns: 64-byte row segments
     static constexpr int TC = 64 / (int)sizeof(V);
-    static constexpr int NT_COLS = (R2 * TC + 31) / 32 * 32;
+    static constexpr int NT_COLS = ((R1 > R2 ? R1 : R2) * TC + 31) / 32 * 32;
     static constexpr size_t SMEM_ROWS = (size_t)L * R2 * LD * sizeof(V), SMEM_COLS = (size_t)R2 * LD * TC * sizeof(V);
 };
 

@@ -56,13 +56,10 @@ __device__ __forceinline__ unsigned operator/(unsigned n, const FastDiv& f) {
 // and the FMA pipe elsewhere (500 = 20 x 25: 3.5 TB/s, 166 us for 144 waves, FMA pipe near half busy).
 // A group of GT threads takes GR rows at a time: one warp where R1 and R2 divide its lanes evenly (256, 512, 1024 and
 // 128 points: no barrier beyond __syncwarp), else a block.
-#ifndef TEST_GT
-#define TEST_GT 128
-#endif
 template <int N> struct RowPlan {
     static constexpr int R1 = TwoPlan<N>::R1, R2 = TwoPlan<N>::R2;
     static constexpr bool EVEN = (32 % R1 == 0) && (32 % R2 == 0), WARP = EVEN || (R2 == 32 && R1 >= 24);
-    static constexpr int GR = EVEN ? 32 / R1 : WARP ? 1 : TEST_GT / R2;
+    static constexpr int GR = EVEN ? 32 / R1 : WARP ? 1 : 128 / R2;
     static constexpr int GT = WARP ? 32 : (GR * R2 + 31) / 32 * 32;
     static constexpr int NT = WARP ? 128 : GT;
     static constexpr int LD = R1 | 1;  // odd: column walks of M touch every bank pair
@@ -215,7 +212,7 @@ template <int N> struct ColPlan {
     static constexpr int TILE = N * TC;  // float2
     static constexpr int NB = (int)((222 * 1024 - 2 * N * sizeof(float2)) / (TILE * sizeof(float2)));
     // threads an SM, by the registers a step-B item needs: 85, 102, 113 or 128 each
-    static constexpr int MAXT = R2 <= 16 ? 768 : R2 <= 20 ? 640 : R2 <= 25 ? 576 : 512;
+    static constexpr int RM = R1 > R2 ? R1 : R2, MAXT = RM <= 16 ? 768 : RM <= 20 ? 640 : RM <= 25 ? 576 : 512;
     static constexpr int subs_of(int nt) { return MAXT / nt < NB - (NB > 3 ? 2 : 1) ? MAXT / nt : NB - (NB > 3 ? 2 : 1); }
     // Threads of a sub-block: the idle share of its rounds of items, weighed against the threads that leaves an SM; the
     // smallest of equals, since more sub-blocks cover each other's barriers (384: 128 threads 77.9 us, 192 threads

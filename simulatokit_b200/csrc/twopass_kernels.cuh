@@ -317,16 +317,20 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
         place(tile_of(i), b, g);
         const int iy = (int)g * TC + c;
         const bool live = iy < ny;
-        // P comes from L2: the first values of step B are asked for before the wave's tile is waited for
+        // P comes from L2: the first values of step B are asked for ahead, at the start of step B, or where registers are
+        // plenty (R2 <= 16) before the wave's tile is waited for (256: 63 -> 59 us for 256 waves; 512 that way 425 -> 452
+        // for 512 waves, 768 166 -> 183 for 64)
+        constexpr bool SOON = R2 <= 16;
         constexpr int EARLY = MODE == 2 ? 0 : R2 <= 16 ? 8 : R2 == 25 ? 8 : R2 / 2;
         [[maybe_unused]] const float2* const P0 = prop + (MODE != 2 && p_row ? (size_t)__ldg(p_row + b) * N * ny : 0) + iy;
         [[maybe_unused]] float2 pe[EARLY > 0 ? EARLY : 1];
-        if constexpr (EARLY > 0) {
+        [[maybe_unused]] auto ask = [&] {
             const float2* p = P0 + (size_t)item * ny;
             const bool on = live && (R1 * TC % NT == 0 || item < R1);
 #pragma unroll
             for (int t = 0; t < EARLY; ++t, p += R1 * ny) pe[t] = on ? __ldg(p) : make_float2(0.0f, 0.0f);
-        }
+        };
+        if constexpr (EARLY > 0 && SOON) ask();
         if (u == 0) {
             if constexpr (MODE == 2) bulk_wait_read();  // this buffer's last tile has left
             else if (!mbar_wait_bounded(&full[s], (i / buffers) & 1)) {
@@ -376,6 +380,7 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
                 for (int t = 0; t < R2; ++t, p += R1 * ny)
                     v[t] = live ? cmul(cmul(__ldg(p), __ldg(x + R1 * t)), y) : make_float2(0.0f, 0.0f);
             } else {
+                if (EARLY > 0 && !SOON && q == 0) ask();
 #pragma unroll
                 for (int j = 0; j < R2; ++j) v[j] = j ? cmul(m[j & 1][j * TC], tw[j * R1 + k]) : m[0][0];
                 dft_reg<R2, -1>(v);

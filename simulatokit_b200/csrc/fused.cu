@@ -2018,7 +2018,6 @@ void probe_scratch(Context& ctx, const std::vector<JobSpec>& jobs, ProbeScratch&
     if (n_max == 0) return;
     sc.spectrum.ensure(n_max * sizeof(float2));
     sc.tmp.ensure(n_max * sizeof(double2));
-    sc.norm.ensure(sizeof(double));
     sc.rx.ensure(nx_max * sizeof(float2));
     sc.ry.ensure(ny_max * sizeof(float2));
     sc.positions.ensure(xy.size() * sizeof(double));

@@ -46,11 +46,6 @@ __device__ __forceinline__ double antialias_at(int ix, int iy, const GridDev g) 
     return 1.0;
 }
 
-__global__ void k_zero_d2(double2* a, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        a[i] = make_double2(0.0, 0.0);
-}
-
 // f(k^2)/S(k) for one element (LobatoParameterization.swift:51-69; ProjectedPotential.swift:130-153).
 __global__ void k_lobato_kernel(double* out, GridDev g, const double* AB, double pi, double pi2) {
     const long long N = (long long)g.nx * g.ny;
@@ -74,22 +69,29 @@ __global__ void k_lobato_kernel(double* out, GridDev g, const double* AB, double
     }
 }
 
-__global__ void k_scatter(double2* D, const int* pix, const double* w, int count) {
+// The merged weights of a batch of delta images (image[i]: the entry's image, first0 the batch's first) into the zeroed D.
+__global__ void k_scatter(double2* D, const int* pix, const double* w, const int* image, int first, int count, int first0,
+                          long long N) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-        D[pix[i]] = make_double2(w[i], 0.0);
+        D[(long long)(image[first + i] - first0) * N + pix[first + i]] = make_double2(w[first + i], 0.0);
 }
 
-// S += sum over the `count` spectra D_q (N apart) of D_q K_{elem[q]}, the elements in the given (increasing Z) order, so
-// each pixel sees the same sequence of additions as one element at a time.
-__global__ void k_accum_spectra(double2* S, const double2* D, const double* K, const int* elem, int count, long long N) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        double2 s = S[i];
-        for (int q = 0; q < count; ++q) {
-            const double k = K[(long long)elem[q] * N + i];
-            const double2 d = D[(long long)q * N + i];
-            s = make_double2(s.x + d.x * k, s.y + d.y * k);
+// Slice g of `slices`: S_g = (more ? S_g : 0) + the sum over its spectra q in [ptr[g], ptr[g + 1]) of D_{q - first0}
+// K_{elem[q]}, the elements in increasing Z, so each pixel sees the same sequence of additions as one element at a time.
+__global__ void k_accum_spectra(double2* S, const double2* D, const double* K, const int* elem, const int* ptr, int slices,
+                                int first0, int more, long long N) {
+    for (int g = blockIdx.y; g < slices; g += gridDim.y) {
+        const int q0 = ptr[g], q1 = ptr[g + 1];
+        double2* const out = S + (long long)g * N;
+        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
+            double2 s = more ? out[i] : make_double2(0.0, 0.0);
+            for (int q = q0; q < q1; ++q) {
+                const double k = K[(long long)elem[q] * N + i];
+                const double2 d = D[(long long)(q - first0) * N + i];
+                s = make_double2(s.x + d.x * k, s.y + d.y * k);
+            }
+            out[i] = s;
         }
-        S[i] = s;
     }
 }
 
@@ -187,6 +189,8 @@ void build_potential_from_atoms(Context& ctx, PotentialImpl& pot, int pi_choice,
     // ProjectedPotential.swift:178-201; merged per pixel as MetalEngine.swift:254-275)
     std::vector<int> pix;
     std::vector<double> wts;
+    std::vector<int> image;  // per entry: its delta image, counted over the (slice, element) groups that have any
+    int images = 0;
     std::vector<long long> group_ptr(1, 0);
     struct Weight {
         int pixel, order;
@@ -225,7 +229,9 @@ void build_potential_from_atoms(Context& ctx, PotentialImpl& pot, int pi_choice,
                 for (; i < entries.size() && entries[i].pixel == p; ++i) sum += entries[i].w;
                 pix.push_back(p);
                 wts.push_back(sum);
+                image.push_back(images);
             }
+            if (!entries.empty()) ++images;
             group_ptr.push_back((long long)pix.size());
         }
     }
@@ -234,9 +240,12 @@ void build_potential_from_atoms(Context& ctx, PotentialImpl& pot, int pi_choice,
     DeviceBuffer& d_w = ctx.pot_w;
     d_pix.ensure(std::max<size_t>(1, pix.size() * sizeof(int)));
     d_w.ensure(std::max<size_t>(1, wts.size() * sizeof(double)));
+    ctx.pot_image.ensure(std::max<size_t>(1, image.size() * sizeof(int)));
     if (!pix.empty()) {
         SIMK_CUDA(cudaMemcpyAsync(d_pix.ptr, pix.data(), pix.size() * sizeof(int), cudaMemcpyHostToDevice, ctx.stream));
         SIMK_CUDA(cudaMemcpyAsync(d_w.ptr, wts.data(), wts.size() * sizeof(double), cudaMemcpyHostToDevice, ctx.stream));
+        SIMK_CUDA(cudaMemcpyAsync(ctx.pot_image.ptr, image.data(), image.size() * sizeof(int), cudaMemcpyHostToDevice,
+                                  ctx.stream));
     }
     DeviceBuffer& kern = ctx.pot_kern;
     DeviceBuffer& ab = ctx.pot_ab;
@@ -275,65 +284,56 @@ void build_potential_from_atoms(Context& ctx, PotentialImpl& pot, int pi_choice,
     DeviceBuffer& d_elem = ctx.pot_elem;
     spec.ensure((size_t)std::min(gmax, std::max(1, S)) * img);
     delta.ensure((size_t)chunk * img);
-    d_elem.ensure((size_t)std::max(1, S * E) * sizeof(int));
-    std::vector<int> present;  // per slice, the elements with atoms in it, in increasing Z; concatenated over slices
-    std::vector<int> present_ptr(1, 0);
+    // per slice, the elements with atoms in it, in increasing Z, concatenated over slices (the images), and where each
+    // image's entries and each slice's images begin: one scatter and one accumulation a group, whatever its images
+    std::vector<int> present, present_ptr(1, 0), entry_ptr(1, 0);
     for (int j = 0; j < S; ++j) {
         for (int e = 0; e < E; ++e)
-            if (group_ptr[j * E + e + 1] > group_ptr[j * E + e]) present.push_back(e);
+            if (group_ptr[j * E + e + 1] > group_ptr[j * E + e]) {
+                present.push_back(e);
+                entry_ptr.push_back((int)group_ptr[j * E + e + 1]);
+            }
         present_ptr.push_back((int)present.size());
     }
-    if (!present.empty())
-        SIMK_CUDA(cudaMemcpyAsync(d_elem.ptr, present.data(), present.size() * sizeof(int), cudaMemcpyHostToDevice,
-                                  ctx.stream));
+    std::vector<int> lists(present);
+    lists.insert(lists.end(), present_ptr.begin(), present_ptr.end());
+    d_elem.ensure(lists.size() * sizeof(int));
+    SIMK_CUDA(cudaMemcpyAsync(d_elem.ptr, lists.data(), lists.size() * sizeof(int), cudaMemcpyHostToDevice, ctx.stream));
+    const int* const elem_of = d_elem.as<int>();
+    const int* const images_of = elem_of + present.size();
     const LinePlan& prow = ctx.plan(g.ny, 64);
     const LinePlan& pcol = ctx.plan(g.nx, 64);
-    // delta image q (of the batch starting at q0) of slice j: its element's atoms scattered with their weights
-    auto scatter = [&](int j, int q_global, int q_local) {
-        const int e = present[q_global];
-        const long long a0 = group_ptr[j * E + e], a1 = group_ptr[j * E + e + 1];
-        k_scatter<<<blocks_for(a1 - a0), 256, 0, ctx.stream>>>(delta.as<double2>() + (long long)q_local * N,
-                                                                d_pix.as<int>() + a0, d_w.as<double>() + a0,
-                                                                (int)(a1 - a0));
+    // the images [q0, q1) transformed in the delta scratch
+    auto transform = [&](int q0, int q1) {
+        SIMK_CUDA(cudaMemsetAsync(delta.ptr, 0, (size_t)(q1 - q0) * img, ctx.stream));
+        const int a0 = entry_ptr[q0], a1 = entry_ptr[q1];
+        k_scatter<<<blocks_for(a1 - a0), 256, 0, ctx.stream>>>(delta.as<double2>(), d_pix.as<int>(), d_w.as<double>(),
+                                                                ctx.pot_image.as<int>(), a0, a1 - a0, q0, N);
+        ++ctx.launches;
+        fft2(prow, pcol, delta.ptr, g.nx, g.ny, q1 - q0, -1, 1.0, ctx.stream, &ctx.launches);
+    };
+    auto accumulate = [&](int slices, const int* ptr, int first0, int more) {
+        const int across = std::min(slices, 65535);
+        k_accum_spectra<<<dim3(std::max(1, std::min(blocks_for(N), 148 * 16 / across + 1)), across), 256, 0, ctx.stream>>>(
+            spec.as<double2>(), delta.as<double2>(), kern.as<double>(), elem_of, ptr, slices, first0, more, N);
         ++ctx.launches;
     };
+    DeviceBuffer part;  // an oversized slice's image range, one batch at a time
     for (int j0 = 0; j0 < S;) {
         int j1 = j0 + 1;
         while (j1 < S && j1 - j0 < gmax && present_ptr[j1 + 1] - present_ptr[j0] <= chunk) ++j1;
-        const int G = j1 - j0;
-        const int imgs = present_ptr[j1] - present_ptr[j0];
-        k_zero_d2<<<blocks_for((long long)G * N), 256, 0, ctx.stream>>>(spec.as<double2>(), (long long)G * N);
-        ++ctx.launches;
-        if (imgs <= chunk) {
-            if (imgs > 0) {
-                k_zero_d2<<<blocks_for((long long)imgs * N), 256, 0, ctx.stream>>>(delta.as<double2>(),
-                                                                                   (long long)imgs * N);
-                ++ctx.launches;
-                for (int j = j0; j < j1; ++j)
-                    for (int q = present_ptr[j]; q < present_ptr[j + 1]; ++q) scatter(j, q, q - present_ptr[j0]);
-                fft2(prow, pcol, delta.ptr, g.nx, g.ny, imgs, -1, 1.0, ctx.stream, &ctx.launches);
-                for (int j = j0; j < j1; ++j) {
-                    const int nq = present_ptr[j + 1] - present_ptr[j];
-                    if (nq == 0) continue;
-                    k_accum_spectra<<<blocks_for(N), 256, 0, ctx.stream>>>(
-                        spec.as<double2>() + (long long)(j - j0) * N,
-                        delta.as<double2>() + (long long)(present_ptr[j] - present_ptr[j0]) * N, kern.as<double>(),
-                        d_elem.as<int>() + present_ptr[j], nq, N);
-                    ++ctx.launches;
-                }
-            }
+        const int G = j1 - j0, q0 = present_ptr[j0], q1 = present_ptr[j1];
+        if (q1 - q0 <= chunk) {
+            if (q1 > q0) transform(q0, q1);
+            accumulate(G, images_of + j0, q0, 0);
         } else {  // G == 1: the slice's images in batches of `chunk`
-            for (int q0 = present_ptr[j0]; q0 < present_ptr[j1]; q0 += chunk) {
-                const int nq = std::min(chunk, present_ptr[j1] - q0);
-                k_zero_d2<<<blocks_for((long long)nq * N), 256, 0, ctx.stream>>>(delta.as<double2>(),
-                                                                                 (long long)nq * N);
-                ++ctx.launches;
-                for (int q = 0; q < nq; ++q) scatter(j0, q0 + q, q);
-                fft2(prow, pcol, delta.ptr, g.nx, g.ny, nq, -1, 1.0, ctx.stream, &ctx.launches);
-                k_accum_spectra<<<blocks_for(N), 256, 0, ctx.stream>>>(spec.as<double2>(), delta.as<double2>(),
-                                                                        kern.as<double>(), d_elem.as<int>() + q0, nq,
-                                                                        N);
-                ++ctx.launches;
+            for (int q = q0; q < q1; q += chunk) {
+                const int range[2] = {q, std::min(q + chunk, q1)};
+                transform(range[0], range[1]);
+                part.ensure(sizeof(range));
+                SIMK_CUDA(cudaStreamSynchronize(ctx.stream));  // the last batch has read its range
+                copy_to_device(part.ptr, range, sizeof(range));
+                accumulate(1, part.as<int>(), q, q > q0);
             }
         }
         fft2(prow, pcol, spec.ptr, g.nx, g.ny, G, +1, 1.0 / (double)N, ctx.stream, &ctx.launches);
@@ -544,18 +544,28 @@ void apply_ctf_device(Context& ctx, const GridGeom& g, double energy, const simk
     }
 }
 
-// One block: the float64 sum of |a|^2 in a fixed order (deterministic).
-__global__ void k_norm2(const double2* a, long long N, double* out) {
-    __shared__ double part[1024];
-    double s = 0.0;
-    for (long long i = threadIdx.x; i < N; i += blockDim.x) s += a[i].x * a[i].x + a[i].y * a[i].y;
+// The float64 sum of |a|^2 in a fixed order (deterministic): block b sums its strided share into out[1 + b], then one
+// block the kNormBlocks shares into out[0]. (One block over everything: 92 us at 768^2, 35 us at 500^2; 6 us now.)
+constexpr int kNormBlocks = 256;
+__device__ __forceinline__ double block_sum(double s) {
+    __shared__ double part[256];
     part[threadIdx.x] = s;
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    for (int w = 128; w > 0; w >>= 1) {
         if ((int)threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *out = part[0];
+    return part[0];
+}
+__global__ void __launch_bounds__(256) k_norm2_shares(const double2* a, long long N, double* out) {
+    double s = 0.0;
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < N; i += kNormBlocks * 256LL) s += a[i].x * a[i].x + a[i].y * a[i].y;
+    s = block_sum(s);
+    if (threadIdx.x == 0) out[1 + blockIdx.x] = s;
+}
+__global__ void __launch_bounds__(256) k_norm2(double* out) {
+    const double s = block_sum(out[1 + threadIdx.x]);
+    if (threadIdx.x == 0) out[0] = s;
 }
 
 __global__ void k_scale_d2(double2* a, long long N, const double* norm2) {
@@ -565,7 +575,7 @@ __global__ void k_scale_d2(double2* a, long long N, const double* norm2) {
 }
 
 namespace {
-// The normalised probe spectrum in float64 into tmp (N double2, norm one double) and as complex64 into out.
+// The normalised probe spectrum in float64 into tmp (N double2, norm 1 + kNormBlocks doubles) and as complex64 into out.
 void probe_spectrum_launch(Context& ctx, const GridGeom& g, const simk_probe& probe, double2* tmp, double* norm,
                            float2* out) {
     SIMK_REQUIRE(std::isfinite(probe.energy) && probe.energy > 0, "the energy must be finite and positive");
@@ -582,10 +592,11 @@ void probe_spectrum_launch(Context& ctx, const GridGeom& g, const simk_probe& pr
     p.day = rsy * 1e3 * p.lambda * 1e-3;
     for (int i = 0; i < 25; ++i) p.ab[i] = probe.aberrations[i];
     k_probe_spectrum<<<blocks_for(N), 256, 0, ctx.stream>>>(tmp, grid_dev(g), p);
-    k_norm2<<<1, 1024, 0, ctx.stream>>>(tmp, N, norm);
+    k_norm2_shares<<<kNormBlocks, 256, 0, ctx.stream>>>(tmp, N, norm);
+    k_norm2<<<1, 256, 0, ctx.stream>>>(norm);
     k_scale_d2<<<blocks_for(N), 256, 0, ctx.stream>>>(tmp, N, norm);
     k_to_float2<<<blocks_for(N), 256, 0, ctx.stream>>>(out, tmp, N);
-    ctx.launches += 4;
+    ctx.launches += 5;
     SIMK_CUDA(cudaGetLastError());
 }
 }  // namespace
@@ -594,7 +605,7 @@ void probe_spectrum_into(Context& ctx, const GridGeom& g, const simk_probe& prob
                          DeviceBuffer& tmp, DeviceBuffer& norm) {
     const long long N = g.count();
     tmp.ensure(N * sizeof(double2));
-    norm.ensure(sizeof(double));
+    norm.ensure((1 + kNormBlocks) * sizeof(double));
     out_f32.ensure(N * sizeof(float2));
     probe_spectrum_launch(ctx, g, probe, tmp.as<double2>(), norm.as<double>(), out_f32.as<float2>());
 }
@@ -602,7 +613,7 @@ void probe_spectrum_into(Context& ctx, const GridGeom& g, const simk_probe& prob
 void probe_spectrum_device(Context& ctx, const GridGeom& g, const simk_probe& probe, DeviceBuffer& out_f32,
                            DeviceBuffer* out_f64) {
     const long long N = g.count();
-    DeviceBuffer tmp(N * sizeof(double2)), norm(sizeof(double));
+    DeviceBuffer tmp(N * sizeof(double2)), norm((1 + kNormBlocks) * sizeof(double));
     out_f32.alloc(N * sizeof(float2));
     probe_spectrum_launch(ctx, g, probe, tmp.as<double2>(), norm.as<double>(), out_f32.as<float2>());
     if (out_f64) {

@@ -645,6 +645,7 @@ __global__ void __launch_bounds__(TC * (N / 8), tc_min_blocks(TC * (N / 8), ENG)
     else if constexpr (ENG == 3)
         eng = tc5_setup<tc5_blocks(N, TC)>(smem_tma + 4 * (size_t)TILE * sizeof(float2), &tmem_slot, &mma_bar, tid,
                                            TC * T, tc5_stack);
+    if constexpr (ENG == 3) tc5_twiddles<N, TC, true>(eng, tw, tid);
     auto issue = [&](unsigned tile, int s) {
         const int b = (int)(tile / tiles_per_wave);
         const int iy0 = (int)(tile - (unsigned)b * tiles_per_wave) * TC;
@@ -742,7 +743,7 @@ __global__ void __launch_bounds__(TC * (N / 8), tc_min_blocks(TC * (N / 8), ENG)
             constexpr int NV = N / 16;
             float2 z[8];
             int ln, i0;
-            bool ok = tc5_fft<N, TC, true, -1, PRE_NONE>(buf, nullptr, 1.0f, tw, eng, tid, z, ln, i0);
+            bool ok = tc5_fft<N, TC, true, -1, PRE_NONE>(buf, nullptr, 1.0f, eng, tid, z, ln, i0);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int o = (i0 + NV * i) * TC + ln;
@@ -750,7 +751,7 @@ __global__ void __launch_bounds__(TC * (N / 8), tc_min_blocks(TC * (N / 8), ENG)
             }
             if constexpr (MODE == 0) {
                 __syncthreads();  // the spectrum times P is in the stage: the inverse transform gathers from it
-                ok = tc5_fft<N, TC, true, +1, PRE_NONE>(buf, nullptr, 1.0f, tw, eng, tid, z, ln, i0) && ok;
+                ok = tc5_fft<N, TC, true, +1, PRE_NONE>(buf, nullptr, 1.0f, eng, tid, z, ln, i0) && ok;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) buf[(i0 + NV * i) * TC + ln] = z[i];
             }
@@ -841,6 +842,7 @@ __global__ void __launch_bounds__(RB * (N / 8), tc_min_blocks(RB * (N / 8), ENG)
     else if constexpr (ENG == 3)
         eng = tc5_setup<tc5_blocks(N, RB)>(smem_rtma + 4 * (size_t)TILE * sizeof(float2), &tmem_slot, &mma_bar, tid,
                                            RB * T, tc5_stack);
+    if constexpr (ENG == 3) tc5_twiddles<N, RB, false>(eng, tw, tid);
     // the finished rows go back by a bulk store from the stage: its wave rows (ENG 0, 3) or its rows of t (ENG 4)
     constexpr bool kStoreFromStage = (ENG == 0 || ENG == 3 || ENG == 4);
     auto issue = [&](int tile, int s) {
@@ -952,7 +954,7 @@ __global__ void __launch_bounds__(RB * (N / 8), tc_min_blocks(RB * (N / 8), ENG)
             int ln, i0;
             bool ok = true;
             if (inv) {
-                ok = tc5_fft<N, RB, false, +1, PRE_NONE>(buf, nullptr, 1.0f, tw, eng, tid, z, ln, i0);
+                ok = tc5_fft<N, RB, false, +1, PRE_NONE>(buf, nullptr, 1.0f, eng, tid, z, ln, i0);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int o = ln * N + i0 + NV * i;
@@ -960,11 +962,11 @@ __global__ void __launch_bounds__(RB * (N / 8), tc_min_blocks(RB * (N / 8), ENG)
                 }
                 if (fwd) {
                     __syncthreads();  // the rows times t are in the stage: the forward transform gathers from them
-                    ok = tc5_fft<N, RB, false, -1, PRE_NONE>(buf, nullptr, 1.0f, tw, eng, tid, z, ln, i0) && ok;
+                    ok = tc5_fft<N, RB, false, -1, PRE_NONE>(buf, nullptr, 1.0f, eng, tid, z, ln, i0) && ok;
                 }
             } else if (fwd) {
-                if (with_t) ok = tc5_fft<N, RB, false, -1, PRE_MUL>(buf, tbuf, scale, tw, eng, tid, z, ln, i0);
-                else ok = tc5_fft<N, RB, false, -1, PRE_SCALE>(buf, nullptr, scale, tw, eng, tid, z, ln, i0);
+                if (with_t) ok = tc5_fft<N, RB, false, -1, PRE_MUL>(buf, tbuf, scale, eng, tid, z, ln, i0);
+                else ok = tc5_fft<N, RB, false, -1, PRE_SCALE>(buf, nullptr, scale, eng, tid, z, ln, i0);
             } else {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -1249,11 +1251,12 @@ bool launch_rows_tma_k(Context& ctx, const RegPlan& p, float2* psi, const float2
     }
 }
 
-// The composite engine's row pass is instantiated per (inverse, forward) pair; the other engines take them at run time.
+// The composite and tcgen05 engines' row passes are instantiated per (inverse, forward) pair, so that each holds only its
+// own path's registers; the other engines take them at run time.
 template <int N, int ENG>
 bool launch_rows_tma(Context& ctx, const RegPlan& p, float2* psi, const float2* tmul, int nx, long long nrows, int inv,
                      int fwd, float scale) {
-    if constexpr (ENG == 4) {
+    if constexpr (ENG == 4 || ENG == 3) {
         switch ((inv ? 1 : 0) | (fwd ? 2 : 0)) {
             case 0: return launch_rows_tma_k<N, ENG, 0>(ctx, p, psi, tmul, nx, nrows, 0, 0, scale);
             case 1: return launch_rows_tma_k<N, ENG, 1>(ctx, p, psi, tmul, nx, nrows, 1, 0, scale);

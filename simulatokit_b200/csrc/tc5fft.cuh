@@ -139,6 +139,8 @@ struct Tc5 {
     uint64_t* bar;     // the MMA completion barrier
     uint32_t phase;    // its next parity
     int stack;         // six stacked products (N = 96, 64, 32) instead of twelve of N = 32
+    // this thread's twiddles of the two radix-16 stages, the same for every tile and both directions (tc5_twiddles)
+    float2 wa[8], wb[8];
 };
 
 // The six B matrices (forward, inverse) x (hi, lo, lo2) into shared memory at `b` by all `nthreads` threads, from
@@ -225,6 +227,22 @@ __device__ __forceinline__ void tc5_read(const Tc5& c, uint32_t taddr, float (&d
     }
 }
 
+// The stages' twiddles of this thread's vector (its mapping as in tc5_fft), kept in registers: read from the table inside
+// the stages, their latency stood in every tile's way (long scoreboard 2.1 of 8 stall cycles an instruction). 512^2 x 256 waves,
+// with the row passes instantiated per (inverse, forward): rows 698 -> 576 us, columns 548 -> 503; 256^2 153 -> 141, 126 ->
+// 121.
+template <int N, int LINES, bool COLS> __device__ __forceinline__ void tc5_twiddles(Tc5& c, const float2* __restrict__ tw, int tid) {
+    constexpr int R = N / 256, NV = N / 16, NSA = R;
+    const int warp = tid >> 5, lane = tid & 31;
+    const int h = (warp >> 2) & 1, v = (warp >> 3) * 128 + (warp & 3) * 32 + lane;
+    const int j = COLS ? v / LINES : v % NV, k = j % NSA, rb = (R == 2) ? (j >> 1) : j;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if constexpr (NSA > 1) c.wa[i] = __ldg(tw + k * (8 * h + i) * (N / (16 * NSA)));
+        c.wb[i] = __ldg(tw + ((R == 2 ? k + 16 * h : 8 * h) + i * NSA) * rb);
+    }
+}
+
 // The tile's line FFT. Thread (warp w, lane l) owns vector v = 128 mb + 32 (w % 4) + l, mb = w / 8, and half h =
 // (w / 4) % 2 of it (inputs r and outputs s in 8 h .. 8 h + 7); v is line v % LINES, vector j = v / LINES of a column
 // tile (neighbouring lanes read neighbouring columns) and line v / NV, j = v % NV of a row tile. The input is read
@@ -235,7 +253,7 @@ __device__ __forceinline__ void tc5_read(const Tc5& c, uint32_t taddr, float (&d
 // its last output, and it does not write `src`. line_out, idx0_out: z[i] is element idx0_out + NV i of line line_out.
 template <int N, int LINES, bool COLS, int DIR, int PRE>
 __device__ __forceinline__ bool tc5_fft(const float2* __restrict__ src, const float2* __restrict__ pre, float scale,
-                                        const float2* __restrict__ tw, Tc5& c, int tid, float2 (&z)[8], int& line_out,
+                                        Tc5& c, int tid, float2 (&z)[8], int& line_out,
                                         int& idx0_out) {
     constexpr int R = N / 256;
     static_assert(R == 1 || R == 2, "tcgen05 line lengths: 256 and 512");
@@ -266,7 +284,6 @@ __device__ __forceinline__ bool tc5_fft(const float2* __restrict__ src, const fl
 
     // ---- stage A: gather (radix-2 first stage folded in for R = 2), twiddle, split, write A rows ----
     {
-        const int k = j % NSA;
         uint32_t hw[8], lw[8], l2w[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -281,7 +298,7 @@ __device__ __forceinline__ bool tc5_fft(const float2* __restrict__ src, const fl
                 x = load(p);
             }
             if constexpr (NSA > 1) {
-                const float2 w = __ldg(tw + k * r * (N / (16 * NSA)));
+                const float2 w = c.wa[i];
                 x = (DIR < 0) ? cmul(x, w) : cmulc(x, w);
             }
             tc5_split3(x, hw[i], lw[i], l2w[i]);
@@ -315,11 +332,10 @@ __device__ __forceinline__ bool tc5_fft(const float2* __restrict__ src, const fl
         constexpr int kRowStep = NSA * (COLS ? LINES : 1);
         uint8_t* p0 = a_blk + (size_t)(vb0 >> 7) * 3 * kTc5Plane + (size_t)(vb0 & 127) * 16 +
                       (size_t)(rb >> 2) * kTc5Lbo + (size_t)(rb & 3) * 4;
-        const float2* w0 = tw + (R == 2 ? (k + 16 * h) : 8 * h) * rb;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             float2 x = make_float2(d[2 * i], d[2 * i + 1]);
-            const float2 w = __ldg(w0 + i * NSA * rb);
+            const float2 w = c.wb[i];
             x = (DIR < 0) ? cmul(x, w) : cmulc(x, w);
             uint32_t hh, ll, l2;
             tc5_split3(x, hh, ll, l2);

@@ -7,6 +7,9 @@
 // The probe is generated inside the first column pass (Psi0 . r_x . r_y -> column IFFT) and the detectors read the
 // last column pass's k-space wave: FFT2(IFFT2(P Phi)) = P Phi, so |FFT2(exit)|^2 = |P Phi|^2 without two transforms.
 //
+// Grid sides from 128 to 1024 with a split N = R1 R2 run the two-pass kernels (twopass_kernels.cuh). The engines in this
+// file take the other sides, the bf16x3 form and the options that name them (column tiles, composite or TMA off).
+//
 // Each line transform is register-resident: with E elements per thread and T = n / E threads per line, thread t holds
 // elements t + T i (i < E). A Stockham pass of radix R (R | E) then reads its butterfly inputs from the thread's own
 // registers, and the last pass writes them back to the same slots, so a transform of P passes exchanges data through
@@ -1355,7 +1358,8 @@ bool cols_ct_tc(Context& ctx, const RegPlan& p, const ColArgs& a, int count, int
         switch (tc) {
             case 2: if (launch_cols_tma<N, 2>(ctx, p, a, count)) return true; break;
             case 4: if (launch_cols_tma<N, 4>(ctx, p, a, count)) return true; break;
-            case 8: if constexpr (8 * (N / 8) <= 1024) { if (launch_cols_tma<N, 8>(ctx, p, a, count)) return true; } break;
+            // (8-column tiles of 512 and 1024 points are the two-pass engine's)
+            case 8: if constexpr (N <= 256) { if (launch_cols_tma<N, 8>(ctx, p, a, count)) return true; } break;
             default: break;
         }
     }
@@ -1479,7 +1483,7 @@ bool cols_cc_tc(Context& ctx, const RegPlan& p, const ColArgs& a, int count) {
     if constexpr (TC * (N / 8) > 1024) {
         return false;
     } else {
-        if constexpr (comp_length(N)) {
+        if constexpr (comp_length(N) && (TC < 8 || N > 1024)) {  // (8 columns up to 1024: the two-pass engine)
             if (ctx.composite && launch_cols_tma<N, TC, 4>(ctx, p, a, count)) return true;
         }
         return launch_cols_tma<N, TC, 2>(ctx, p, a, count);
@@ -1528,11 +1532,8 @@ bool rows_two(Context& ctx, const RegPlan& p, float2* psi, const float2* tmul, i
 // register engine's tile, 16 does.
 int two_tile(int n) { return n == 256 ? 16 : 8; }
 
-// Columns of 128 points stay on the register engine: its 4-column tiles took 41.5 us for 512 waves and 7.0 us for one,
-// the two-pass engine 45.2 and 8.5 (at 192 points 74.9 against the runtime plan's several times that; at 256 61.8
-// against 68.3 for 256 waves).
 bool cols_two_wanted(const Context& ctx, int n) {
-    return n > 128 && two_wanted(ctx, n) && (ctx.col_tile == 0 || ctx.col_tile == two_tile(n));
+    return n > kTwoColsAbove && two_wanted(ctx, n) && (ctx.col_tile == 0 || ctx.col_tile == two_tile(n));
 }
 
 bool cols_two(Context& ctx, const RegPlan& p, const ColArgs& a, int count) {

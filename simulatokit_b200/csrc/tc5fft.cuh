@@ -261,7 +261,7 @@ __device__ __forceinline__ bool tc5_fft(const float2* __restrict__ src, const fl
     constexpr int V = LINES * NV;        // vectors in the tile
     constexpr int MB = V / 128;
     static_assert(V % 128 == 0, "blocks of 128 vectors");
-    constexpr int NSA = R, NSB = 16 * R;  // the two radix-16 stages' spans
+    [[maybe_unused]] constexpr int NSA = R, NSB = 16 * R;  // the two radix-16 stages' spans
     const int warp = tid >> 5, lane = tid & 31;
     const int mb = warp >> 3, h = (warp >> 2) & 1, q = warp & 3;
     const int v = mb * 128 + q * 32 + lane;

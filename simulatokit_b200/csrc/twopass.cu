@@ -64,8 +64,10 @@ bool twopass_rows(Context& ctx, float2* psi, const float2* tmul, int nx, int ny,
 
 bool twopass_cols(Context& ctx, int nx, const TwoPassCols& a, int* groups) {
     switch (nx) {
-#define SIMK_TWO_PLAN(n, r1, r2) \
-    case n: return launch_two_cols<n>(ctx, twopass_table(ctx, n), a, groups);
+#define SIMK_TWO_PLAN(n, r1, r2)                                                                               \
+    case n:                                                                                                    \
+        if constexpr (n > kTwoColsAbove) return launch_two_cols<n>(ctx, twopass_table(ctx, n), a, groups);     \
+        else return false;
 #include "twopass_plans.inc"
 #undef SIMK_TWO_PLAN
         default: return false;

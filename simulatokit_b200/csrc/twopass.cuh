@@ -19,6 +19,10 @@ struct TwoPassCols {
     const FusedDetect* det = nullptr;
 };
 
+// Columns of up to this length stay on the register engine: at 128 points its 4-column tiles took 41.5 us for 512 waves
+// and 7.0 us for one, the two-pass engine 45.2 and 8.5; at 256 68.3 against 61.8 for 256 waves.
+constexpr int kTwoColsAbove = 128;
+
 // Whether lines of n points have a plan here.
 bool twopass_length(int n);
 // The plan's twiddle table of n, created on first use (allocates and copies: not inside a stream capture).
@@ -26,7 +30,7 @@ const float2* twopass_table(Context& ctx, int n);
 // The row pass over nrows = count nx rows of ny points: [inverse], x t x scale, [forward]. False: no plan for ny.
 bool twopass_rows(Context& ctx, float2* psi, const float2* tmul, int nx, int ny, long long nrows, int inv, int fwd,
                   float scale);
-// The column pass over lines of nx points; with mode 3 *groups receives the column groups of the partial sums.
+// The column pass over lines of nx > kTwoColsAbove points (false otherwise, or without a plan); with mode 3 *groups receives the column groups of the partial sums.
 bool twopass_cols(Context& ctx, int nx, const TwoPassCols& a, int* groups);
 
 }  // namespace simk

@@ -9,93 +9,100 @@ namespace simk {
 
 // ---- freed device blocks ---------------------------------------------------------------------------------------------
 // cudaMalloc and cudaFree of a call's temporaries and of a potential's slices took 50-300 us each, half of a small HRTEM
-// image. A freed block is kept (per device, at most kKept bytes in all, the oldest going first) and handed out again to
-// a request it fits within a quarter. Every block comes back only after the device has finished everything queued, as
-// cudaFree waits, so any stream and thread may take it next. When the last context goes, so do the blocks.
+// image, and now and then a fresh block tens of ms on a busy host. (A list of freed blocks that were never split or joined
+// missed on each new potential: 512^2 scan, first pass 154-215 ms, now 154; 768^2 phonons 18-36, now 17; a new job table
+// 42, now 34.) Blocks of up to kLargest come from one memory pool a device, which splits and joins what it holds and
+// grows by whole chunks; at most kKept bytes beyond the blocks in use stay there. Every block goes back only after the
+// device has finished everything queued, as cudaFree waits, and the pool's stream is idle when one is handed out, so any
+// stream and thread may take it next. When the last context goes, so does what the pool holds free.
 namespace {
 constexpr size_t kKept = 512u << 20;
-struct Block {
-    void* ptr;
-    size_t bytes;
-};
-struct DeviceBlocks {
-    std::vector<Block> kept;  // oldest first
-    size_t bytes = 0;
+constexpr size_t kLargest = 256u << 20;
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;  // orders the pool's operations
+    size_t live = 0;                // bytes handed out
     int contexts = 0;
 };
-std::mutex g_blocks_mutex;
-std::map<int, DeviceBlocks>& device_blocks() {
-    static auto* m = new std::map<int, DeviceBlocks>();  // never destroyed: buffers may be released at exit
-    return *m;
+std::mutex g_pools_mutex;
+DevicePool& device_pool(int device) {
+    static auto* m = new std::map<int, DevicePool>();  // never destroyed: buffers may be released at exit
+    return (*m)[device];
 }
-void drop_all(DeviceBlocks& d) {
-    for (Block& b : d.kept) cudaFree(b.ptr);
-    d.kept.clear();
-    d.bytes = 0;
+void open_pool(DevicePool& d, int device) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    SIMK_CUDA(cudaMemPoolCreate(&d.pool, &props));
+    unsigned long long hold = ~0ULL;  // what stays is bounded in device_free
+    SIMK_CUDA(cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &hold));
+    SIMK_CUDA(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking));
+}
+cudaError_t pool_alloc(DevicePool& d, void** p, size_t n) {
+    const cudaError_t e = cudaMallocFromPoolAsync(p, n, d.pool, d.stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(d.stream) : e;
 }
 }  // namespace
 
 void* device_alloc(size_t n, size_t* got, int* device) {
     n = (n + 511) / 512 * 512;
     SIMK_CUDA(cudaGetDevice(device));
-    std::lock_guard<std::mutex> lk(g_blocks_mutex);
-    DeviceBlocks& d = device_blocks()[*device];
-    size_t best = d.kept.size();
-    for (size_t i = 0; i < d.kept.size(); ++i) {
-        const size_t b = d.kept[i].bytes;
-        if (b >= n && b <= n + std::max<size_t>(n / 4, 4096) && (best == d.kept.size() || b < d.kept[best].bytes)) best = i;
-    }
-    if (best < d.kept.size()) {
-        const Block b = d.kept[best];
-        d.kept.erase(d.kept.begin() + best);
-        d.bytes -= b.bytes;
-        *got = b.bytes;
-        return b.ptr;
-    }
+    std::lock_guard<std::mutex> lk(g_pools_mutex);
+    DevicePool& d = device_pool(*device);
+    if (!d.pool) open_pool(d, *device);
+    auto take = [&](void** p) { return n > kLargest ? cudaMalloc(p, n) : pool_alloc(d, p, n); };
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, n);
-    if (e == cudaErrorMemoryAllocation && !d.kept.empty()) {
+    cudaError_t e = take(&p);
+    if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        drop_all(d);
-        e = cudaMalloc(&p, n);
+        cudaMemPoolTrimTo(d.pool, 0);
+        e = take(&p);
     }
     check_cuda(e, "cudaMalloc");
+    if (n <= kLargest) d.live += n;
     *got = n;
     return p;
 }
 
 void device_free(void* p, size_t bytes, int device) {
     if (!p) return;
+    if (bytes > kLargest) {
+        cudaFree(p);
+        return;
+    }
     int current = device;
     cudaGetDevice(&current);
     if (current != device) cudaSetDevice(device);
+    cudaDeviceSynchronize();
     {
-        std::lock_guard<std::mutex> lk(g_blocks_mutex);
-        DeviceBlocks& d = device_blocks()[device];
-        if (d.contexts == 0 || bytes > kKept / 2 || cudaDeviceSynchronize() != cudaSuccess) {
-            cudaFree(p);
-        } else {
-            d.kept.push_back({p, bytes});
-            d.bytes += bytes;
-            while (d.bytes > kKept) {
-                cudaFree(d.kept.front().ptr);
-                d.bytes -= d.kept.front().bytes;
-                d.kept.erase(d.kept.begin());
-            }
+        std::lock_guard<std::mutex> lk(g_pools_mutex);
+        DevicePool& d = device_pool(device);
+        cudaFreeAsync(p, d.stream);
+        d.live -= bytes;
+        unsigned long long held = 0;
+        cudaMemPoolGetAttribute(d.pool, cudaMemPoolAttrReservedMemCurrent, &held);
+        const size_t keep = d.live + (d.contexts ? kKept : 0);
+        if (held > keep) {
+            cudaStreamSynchronize(d.stream);
+            cudaMemPoolTrimTo(d.pool, keep);
         }
     }
     if (current != device) cudaSetDevice(current);
 }
 
 void device_context_made(int device) {
-    std::lock_guard<std::mutex> lk(g_blocks_mutex);
-    ++device_blocks()[device].contexts;
+    std::lock_guard<std::mutex> lk(g_pools_mutex);
+    ++device_pool(device).contexts;
 }
 
 void device_context_gone(int device) {
-    std::lock_guard<std::mutex> lk(g_blocks_mutex);
-    DeviceBlocks& d = device_blocks()[device];
-    if (--d.contexts == 0) drop_all(d);
+    std::lock_guard<std::mutex> lk(g_pools_mutex);
+    DevicePool& d = device_pool(device);
+    if (--d.contexts == 0 && d.pool) {
+        cudaStreamSynchronize(d.stream);
+        cudaMemPoolTrimTo(d.pool, 0);
+    }
 }
 
 // ---- pinned staging --------------------------------------------------------------------------------------------------

@@ -1515,9 +1515,10 @@ bool cols_cc(Context& ctx, const RegPlan& p, const ColArgs& a, int count) {
 }
 
 // ---- the two-pass engine (twopass.cuh): one exchange a transform, wherever the length has a plan and the settings ask
-// for no other engine. Measured against the engines it replaced (one box, us a launch, rows | columns): 512^2 x 512 waves
-// 516 -> 420 | 488 -> 440; 1024^2 x 128 671 -> 438 | 735 -> 556; 768^2 x 64 249 -> 148 | 246 -> 166; 500^2 x 144
-// 691 -> 166 | 632 -> 170; 256^2 x 256 69 -> 52 | 68 -> 62 --------------------------------------------------------------
+// for no other engine. Measured against the engines it replaced (one box, us a launch, rows | columns, means over a
+// 6-slice scan's launches, probe generation and detection among the columns'): 512^2 x 512 waves 516 -> 420 | 488 -> 437;
+// 1024^2 x 128 671 -> 438 | 735 -> 544; 768^2 x 64 249 -> 148 | 246 -> 172; 500^2 x 144 691 -> 166 | 632 -> 167;
+// 256^2 x 256 69 -> 52 | 68 -> 60 -------------------------------------------------------------------------------------
 bool two_wanted(const Context& ctx, int n) {
     if (!ctx.tma || !twopass_length(n)) return false;
     return comp_length(n) ? ctx.composite != 0 : true;

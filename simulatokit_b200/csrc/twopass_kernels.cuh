@@ -200,8 +200,8 @@ __global__ void __launch_bounds__(RowPlan<N>::NT, RowPlan<N>::BLOCKS)
 // to SUBS of them, which synchronise apart and share a ring of NB tile buffers: tile i of the block is in buffer i % NB
 // and belongs to sub-block i % SUBS. TMA brings a tile in and takes it out; the load of tile i + NB is issued by the
 // sub-block that had tile i, once the store of tile i has read its buffer (asked for in the middle of its next tile).
-// Bound at 512 by the latency of a tile's three steps at four warps a scheduler (4.4-4.7 TB/s, 421-450 us for 512 waves;
-// FMA pipe and issue near half busy). Tiles loaded and stored from registers instead, without TMA: 541 us, most of it
+// Bound at 512 by the latency of a tile's three steps at four warps a scheduler (512 waves: 505 us between two slices,
+// 4.25 TB/s; 437 us the mean of a 6-slice scan's launches, as the times below; FMA pipe and issue near half busy). Tiles loaded and stored from registers instead, without TMA: 541 us, most of it
 // the loads' latency; tiles of 16 columns that way 550 us; P's first values asked for in step B 482 us, before the
 // tile's wait 440 us. Programmatic dependent launch of the passes cost 4 % at 512^2 (5 % at 256^2) and is not used.
 // All three steps work in place: step A's value (j, k) lies in the row j + R2 k that item j owns, with the rows of

@@ -183,7 +183,7 @@ struct Context {
     HostStage stage;  // pinned halves between split float64 host arrays and complex64 device arrays
     DeviceBuffer lobato_elements;  // the scaled Lobato parameters of Z = 1 .. 103
     DeviceBuffer evaluate_work;    // the surrogate's queries, their full projections and results
-    std::map<int, DeviceBuffer> twopass_tables;  // the two-pass engine's twiddles by line length
+    std::map<std::pair<int, long long>, DeviceBuffer> twopass_tables;  // the two-pass engine's, by length and divisor
     std::map<std::tuple<int, int, double, double, double, double, double, double>, std::unique_ptr<Propagator>> props;
     // workspaces
     DeviceBuffer work_a, work_b, work_c, rx, ry, positions, partial;

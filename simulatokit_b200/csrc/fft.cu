@@ -4,7 +4,6 @@
 #include <algorithm>
 #include <complex>
 
-#include "dftreg.cuh"
 #include "linefft.cuh"
 
 namespace simk {
@@ -137,16 +136,15 @@ std::unique_ptr<LinePlan> make_line_plan(int n, int precision) {
     else upload_complex<float2>(p->tw, tw);
     // the one-exchange transforms: the lengths with a plan, and Bluestein's work lengths with one
     if (const int r1 = line_first_radix(p->m); r1 && (!p->bluestein || line_bluestein_length(p->m))) {
-        std::vector<std::complex<double>> t(p->m);
-        for (int i = 0; i < p->m; ++i) {
-            t[i] = tw[(long long)(i / r1) * (i % r1) % p->m];
-            if (precision != 64 && t[i].real() != 0.0 && t[i].imag() != 0.0) {  // on the unit circle as floats (dftreg.cuh)
-                const UnitPair w = unit_pair(t[i].real(), t[i].imag());
-                t[i] = {w.c, w.s};
-            }
+        if (precision == 64) {
+            std::vector<std::complex<double>> t(p->m);
+            for (int i = 0; i < p->m; ++i) t[i] = tw[(long long)(i / r1) * (i % r1) % p->m];
+            upload_complex<double2>(p->table, t);
+        } else {
+            const std::vector<float2> t = line_table(p->m, r1);
+            p->table.alloc(t.size() * sizeof(float2));
+            copy_to_device(p->table.ptr, t.data(), t.size() * sizeof(float2));
         }
-        if (precision == 64) upload_complex<double2>(p->table, t);
-        else upload_complex<float2>(p->table, t);
     }
     // cos/sin tables of the generic radices
     std::vector<double> rc, rs;

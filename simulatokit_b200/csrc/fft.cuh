@@ -5,7 +5,8 @@
 // inverse with e^{+2 pi i jk/n}; the caller applies 1/(nx ny). The Stockham autosort pass with radix R after Ns
 // points have been combined reads v[r] = a[j + r n/R], twiddles v[r] by W_n^{(j mod Ns) r n/(Ns R)}, takes the
 // R-point DFT and writes b[(j - j mod Ns) R + j mod Ns + r Ns]. Twiddles come from tables computed in float64 from
-// exact integer phases (as MixedRadixPlan.swift:72-99 does) and rounded once.
+// exact integer phases (as MixedRadixPlan.swift:72-99 does) and rounded once (the one-exchange transforms' float32 tables
+// are line_table's, linefft.cu).
 #pragma once
 
 #include "common.cuh"

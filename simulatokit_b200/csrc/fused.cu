@@ -1085,10 +1085,14 @@ RegChoice choose(int n) {
     return best;
 }
 
-RegPlan reg_plan(Context& ctx, int n) {
+// The plan of n; as columns of an n x other grid with `other` given.
+RegPlan reg_plan(Context& ctx, int n, int other = 0) {
     RegChoice ch = choose(n);
     SIMK_REQUIRE(ch.E != 0 || (ctx.tma && twopass_length(n)), "no register FFT plan for length " + std::to_string(n));
-    if (twopass_length(n)) twopass_table(ctx, n);  // created here, before a capture
+    if (twopass_length(n)) {  // created here, before a capture
+        twopass_table(ctx, n);
+        if (other > 0) twopass_table(ctx, n, (long long)n * other);
+    }
     RegPlan p{};
     p.n = n;
     p.E = ch.E;  // 0: only the two-pass engine takes the length
@@ -1543,7 +1547,6 @@ bool cols_two(Context& ctx, const RegPlan& p, const ColArgs& a, int count) {
     TwoPassCols c;
     c.psi = a.psi;
     c.P = a.P;
-    c.pscale = a.pscale;
     c.mode = a.mode;
     c.ny = a.ny;
     c.count = count;
@@ -1744,7 +1747,7 @@ int propagate_fused_eager(Context& ctx, PotentialImpl& pot, double energy, doubl
     const GridGeom& g = pot.g;
     const long long N = g.count();
     const RegPlan prow = reg_plan(ctx, g.ny);
-    const RegPlan pcol = reg_plan(ctx, g.nx);
+    const RegPlan pcol = reg_plan(ctx, g.nx, g.ny);
     const int S = pot.n_slices();
     const float invN = 1.0f / (float)N;
     for (int j = 0; j < S; ++j) {
@@ -1788,7 +1791,7 @@ int exit_spectra_fused(Context& ctx, PotentialImpl& pot, const simk_probe& probe
     const GridGeom& g = pot.g;
     float2* psi = ctx.work_a.as<float2>();
     launch_ramps(ctx, g, positions_dev, first, b, ctx.rx.as<float2>(), ctx.ry.as<float2>());
-    const RegPlan pcol = reg_plan(ctx, g.nx);
+    const RegPlan pcol = reg_plan(ctx, g.nx, g.ny);
     ColArgs a{};
     a.psi = psi;
     a.mode = 2;
@@ -1848,7 +1851,7 @@ Context::Tuned autotune(Context& ctx, PotentialImpl& pot, double energy, double 
     cap = std::max(1LL, std::min(cap, 1024LL));  // per grid, not per call: the caller's batches cap themselves
     (void)max_waves;
     const RegPlan prw = reg_plan(ctx, g.ny);
-    const RegPlan pcl = reg_plan(ctx, g.nx);
+    const RegPlan pcl = reg_plan(ctx, g.nx, g.ny);
     const Propagator& P = ctx.propagator(g, energy, pot.dz[0], tx, ty);
     DeviceBuffer buf((size_t)cap * N * sizeof(float2));
     SIMK_CUDA(cudaMemsetAsync(buf.ptr, 0, (size_t)cap * N * sizeof(float2), ctx.stream));
@@ -2303,7 +2306,7 @@ void run_job_table(Context& ctx, const std::vector<JobSpec>& jobs, double* done_
             }
             // what the launches create on first use exists before a capture: the plans and the error flag
             for (auto& gr : runs) {
-                reg_plan(ctx, gr.nx);
+                reg_plan(ctx, gr.nx, gr.ny);
                 reg_plan(ctx, gr.ny);
             }
             ensure_err_flag(ctx);
@@ -2333,7 +2336,7 @@ void run_job_table(Context& ctx, const std::vector<JobSpec>& jobs, double* done_
                     };
                     const int A = active(s);
                     const RegPlan prw = reg_plan(ctx, gr.ny);
-                    const RegPlan pcl = reg_plan(ctx, gr.nx);
+                    const RegPlan pcl = reg_plan(ctx, gr.nx, gr.ny);
                     float2* psi = gr.waves.as<float2>();
                     ctx.wave_t = gr.dt.as<const float2*>() + (size_t)s * G;
                     ctx.wave_p = gr.dp.as<int>() + (size_t)s * G;

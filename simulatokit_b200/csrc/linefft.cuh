@@ -1,6 +1,8 @@
 // linefft.cuh -- batched line transforms with one exchange (kernels in linefft_kernels.cuh): what fft.cu dispatches to.
 #pragma once
 
+#include <vector>
+
 #include "common.cuh"
 
 namespace simk {
@@ -18,6 +20,8 @@ template <typename V> struct LineArgs {
 
 template <int N, bool BLUE, typename V> void launch_line(const LineArgs<V>& a, bool columns, cudaStream_t stream);
 
+// The float32 twiddles W_n^{jk} of a plan n = r1 r2, times `scale`, at j r1 + k.
+std::vector<float2> line_table(int n, int r1, double scale = 1.0);
 // R1 of the plan of N points, 0 where there is none; whether Bluestein's work length N is taken.
 int line_first_radix(int N);
 bool line_bluestein_length(int N);

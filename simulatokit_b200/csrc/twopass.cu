@@ -1,7 +1,7 @@
 // twopass.cu -- the two-pass engine's tables and its dispatch on the line length.
 #include "twopass.cuh"
 
-#include "dftreg.cuh"
+#include "linefft.cuh"
 
 namespace simk {
 
@@ -31,18 +31,12 @@ int first_radix(int n) {
 
 bool twopass_length(int n) { return first_radix(n) != 0; }
 
-const float2* twopass_table(Context& ctx, int n) {
-    DeviceBuffer& buf = ctx.twopass_tables[n];
+const float2* twopass_table(Context& ctx, int n, long long points) {
+    DeviceBuffer& buf = ctx.twopass_tables[{n, points}];
     if (!buf.ptr) {
         const int r1 = first_radix(n);
         SIMK_REQUIRE(r1 != 0, "no two-pass plan for length " + std::to_string(n));
-        std::vector<float2> h(n);  // entry j R1 + k: e^{-2 pi i j k / n}
-        for (int i = 0; i < n; ++i) {
-            double s, c;
-            host_sincospi(-2.0 * (double)((long long)(i / r1) * (i % r1) % n) / (double)n, &s, &c);
-            const UnitPair w = (c == 0.0 || s == 0.0) ? UnitPair{c, s} : unit_pair(c, s);
-            h[i] = make_float2((float)w.c, (float)w.s);
-        }
+        const std::vector<float2> h = line_table(n, r1, 1.0 / (double)points);
         DeviceBuffer made(n * sizeof(float2));
         copy_to_device(made.ptr, h.data(), n * sizeof(float2));
         buf = std::move(made);

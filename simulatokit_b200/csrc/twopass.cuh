@@ -9,8 +9,7 @@ namespace simk {
 struct TwoPassCols {
     float2* psi = nullptr;
     const float2* P = nullptr;
-    float pscale = 1.0f;
-    int mode = 0;  // 0: FFT, x P, IFFT; 1: FFT, x P; 2: the probes' spectrum, IFFT; 3: as 1, with the detection
+    int mode = 0;  // 0: FFT, x P, IFFT / (nx ny); 1: FFT, x P; 2: the probes' spectrum, IFFT; 3: as 1, with the detection
     int ny = 0, count = 0;
     const float2* spectrum = nullptr;
     const float2* rx = nullptr;
@@ -25,8 +24,9 @@ constexpr int kTwoColsAbove = 128;
 
 // Whether lines of n points have a plan here.
 bool twopass_length(int n);
-// The plan's twiddle table of n, created on first use (allocates and copies: not inside a stream capture).
-const float2* twopass_table(Context& ctx, int n);
+// The plan's twiddle table of n divided by `points` (the inverse transform's 1 / (nx ny) in the columns' way back), created
+// on first use (allocates and copies: not inside a stream capture).
+const float2* twopass_table(Context& ctx, int n, long long points = 1);
 // The row pass over nrows = count nx rows of ny points: [inverse], x t x scale, [forward]. False: no plan for ny.
 bool twopass_rows(Context& ctx, float2* psi, const float2* tmul, int nx, int ny, long long nrows, int inv, int fwd,
                   float scale);

@@ -256,7 +256,8 @@ struct TileOrder {
 template <int N, int MODE>
 __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
     two_cols(const __grid_constant__ CUtensorMap map, float2* __restrict__ psi, const float2* __restrict__ prop,
-             const float2* __restrict__ table, float pscale, int ny, TileOrder order, int buffers, int* err,
+             const float2* __restrict__ table, const float2* __restrict__ back, float scale, float rest, int ny,
+             TileOrder order, int buffers, int* err,
              const int* __restrict__ p_row, const float2* __restrict__ rx, const float2* __restrict__ ry, TwoDetect det) {
     using P = ColPlan<N>;
     constexpr int R1 = P::R1, R2 = P::R2, TC = P::TC, NT = P::NT, QA = P::QA, QB = P::QB, TILE = P::TILE,
@@ -265,8 +266,8 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
     extern __shared__ __align__(128) float2 smem_two_cols[];
     __shared__ __align__(8) uint64_t full[P::NB];
     __shared__ int failed[P::SUBS], issued[P::NB];
-    // W_N^{jk}, and for the way back the same times pscale (so that scaling costs nothing: every value but j = 0 takes a
-    // twiddle)
+    // W_N^{jk}, and for the way back the same divided by nx ny (so that scaling costs nothing: every value but j = 0
+    // takes a twiddle)
     float2* const tw = smem_two_cols + buffers * TILE;
     float2* const tw_back = tw + N;
     const unsigned subs = order.subs.d;
@@ -304,9 +305,8 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
             for (int i = 0; i < buffers; ++i) issue(i);
     }
     for (int i = tid; i < N; i += blockDim.x) {
-        const float2 w = __ldg(table + i);
-        tw[i] = w;
-        tw_back[i] = w * pscale;
+        tw[i] = __ldg(table + i);
+        if constexpr (MODE == 0 || MODE == 2) tw_back[i] = __ldg(back + i);
     }
     __syncthreads();
     const int c = u % TC, item = u / TC;
@@ -394,15 +394,17 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
                         p += R1 * ny;
                     }
                 }
-                if (MODE != 0 && pscale != 1.0f) {
-#pragma unroll
-                    for (int t = 0; t < R2; ++t) v[t] = v[t] * pscale;
-                }
             }
             if constexpr (MODE == 0 || MODE == 2) {
                 dft_reg<R2, +1>(v);
 #pragma unroll
-                for (int j = 0; j < R2; ++j) m[j & 1][j * TC] = j ? cmulc(v[j], tw_back[j * R1 + k]) : v[0] * pscale;
+                for (int j = 0; j < R2; ++j) {
+                    // (j = 0 has no twiddle: scale + rest is 1 / (nx ny))
+                    m[j & 1][j * TC] = j           ? cmulc(v[j], tw_back[j * R1 + k])
+                                       : MODE == 0 ? make_float2(fmaf(v[0].x, scale, v[0].x * rest),
+                                                                 fmaf(v[0].y, scale, v[0].y * rest))
+                                                   : v[0];
+                }
             } else {
                 if (live && (MODE == 1 || det.store)) {
                     float2* out = psi + ((size_t)b * N + k) * ny + iy;
@@ -542,9 +544,12 @@ template <int N, int MODE> bool launch_two_cols_m(Context& ctx, const float2* ta
     order.groups = (unsigned)g;
     order.waves = (unsigned)(a.count / subs * subs);
     order.tiles = (unsigned)tiles;
+    const double inverse = MODE == 0 ? 1.0 / ((double)N * a.ny) : 1.0;
+    const float scale = (float)inverse;
+    const float2* const back = MODE == 0 ? twopass_table(ctx, N, (long long)N * a.ny) : table;
     const CUtensorMap map = encode_tensor_map_2d(a.psi, 2ULL * a.ny, (unsigned long long)a.count * N, 2 * P::TC, P::BOXH);
     two_cols<N, MODE><<<grid, P::NT * subs, P::smem(buffers), ctx.stream>>>(
-        map, a.psi, MODE == 2 ? a.spectrum : a.P, table, a.pscale, a.ny, order, buffers,
+        map, a.psi, MODE == 2 ? a.spectrum : a.P, table, back, scale, (float)(inverse - (double)scale), a.ny, order, buffers,
         ctx.err_flag.as<int>(), a.p_row, a.rx, a.ry, d);
     SIMK_CUDA(cudaGetLastError());
     ++ctx.launches;

@@ -149,7 +149,10 @@ void scan_device(Context& ctx, const simk_probe& probe, const std::vector<Potent
                        key_bytes(dets, sizeof(simk_detector) * (size_t)n_det);
     auto dit = ctx.detector_plans.find(dkey);
     if (dit == ctx.detector_plans.end()) {
-        if (ctx.detector_plans.size() > 64) ctx.detector_plans.clear();
+        if (ctx.detector_plans.size() > 64) {
+            ctx.drop_graphs();  // their launches read the plans' lists, and their keys hold the plans' addresses
+            ctx.detector_plans.clear();
+        }
         dit = ctx.detector_plans.emplace(dkey, build_detector_plan(ctx, g, probe.energy, dets, n_det)).first;
     }
     DetectorPlan* dplan = dit->second.get();

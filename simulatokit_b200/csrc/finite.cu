@@ -158,12 +158,17 @@ __global__ void k_finite_points(const int* __restrict__ elem, const double* __re
 // P_inf(rho) = 2 sum_t [2 A/B K0(x) + A rho K1(x)], x = B rho, the full projection of the potential. With
 // K_nu(x) = int_0^inf e^{-x cosh u} cosh(nu u) du each term is int e^{-x cosh u} (2 A/B + A rho cosh u) du, an integrand
 // analytic in |Im u| < pi/2 and, for large x, a Gaussian of width 1/sqrt(x): the trapezoidal rule with step
-// min(0.22, 0.65 / sqrt(x)) leaves less than 1e-15 of it, in 12 to 40 points (against SciPy's K0 and K1: 7e-15 up to
-// x = 30, 7e-14 at 260, the rounding of x cosh u).
+// min(0.22, 0.65 / sqrt(x)) leaves less than 1e-15 of it, in 12 points at x = 10, 21 at 1, 42 at 0.01 and 104 at 1e-8
+// (against SciPy's K0 and K1: 7e-15 up to x = 30, 7e-14 at 260, the rounding of x cosh u). Below 1e-8 the first terms of
+// K0 and K1 are all of them in float64.
 __device__ double infinite_profile_dev(const ElementAB& e, double rho) {
     double total = 0.0;
     for (int t = 0; t < 5; ++t) {
         const double x = e.B[t] * rho, a = 2.0 * e.A[t] / e.B[t], b = e.A[t] * rho;
+        if (x < 1e-8) {
+            total += a * (-log(0.5 * x) - 0.57721566490153286061) + b / x;
+            continue;
+        }
         const double h = fmin(0.22, 0.65 * rsqrt(x)), step = 2.0 * cosh(h);
         double before = 0.5 * step, c = 1.0;  // cosh((k - 1) h), cosh(k h)
         double s = 0.5 * exp(-x) * (a + b);
@@ -283,6 +288,12 @@ void finite_profiles_quadrature(Context& ctx, const FiniteDevice& d, long long n
                                                                       table);
     SIMK_CUDA(cudaGetLastError());
     ++ctx.launches;
+}
+
+bool infinite_in_reach(int z, double rho) {
+    if (rho <= 6000.0) return true;  // no B is above 990
+    const ElementAB e = element_ab(z);
+    return *std::max_element(e.B, e.B + 5) * rho <= 6000684.0;
 }
 
 void infinite_points(Context& ctx, int n, const int* z_dev, const double* rho_dev, double* out_dev) {

@@ -47,6 +47,9 @@ void finite_profiles_quadrature(Context& ctx, const FiniteDevice& d, long long n
 // The full projection P_inf(rho) = 2 sum_i [2 A_i/B_i K0(B_i rho) + A_i rho K1(B_i rho)] at n points (atomic number 1 to
 // 103, rho > 0), float64: on device arrays, or from and to the host.
 void infinite_points(Context& ctx, int n, const int* z_dev, const double* rho_dev, double* out_dev);
+// Whether the radius is one of a full projection: finite, and B rho up to 6,000,684 for every term (all far past where it
+// underflows to 0; the Bessel functions of the C++ library end there, and such radii are refused).
+bool infinite_in_reach(int z, double rho);
 std::vector<double> infinite_profiles(Context& ctx, const std::vector<int>& z, const std::vector<double>& rho);
 void finite_points(Context& ctx, const ElementAB* ab_dev, int n, const int* elem_dev, const double* rho_dev,
                    const double* zl_dev, const double* zu_dev, double* out_dev);

@@ -56,6 +56,15 @@ GridGeom geom_of(const simk_grid* g) {
 
 void activate(Context& c) { SIMK_CUDA(cudaSetDevice(c.device)); }
 
+// For calls that return waves to the host. They end in a wait, which a capture of the user's refuses, but by then what they
+// prepare (a potential's transmissions) has only been recorded, and the calls after it would take it for done.
+void refuse_capture(Context& c) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    SIMK_CUDA(cudaStreamIsCapturing(c.stream, &s));
+    if (s != cudaStreamCaptureStatusNone)
+        throw Error(SIMK_ERR_CUDA, "a call that returns host arrays cannot be captured");
+}
+
 std::vector<double> checked_thickness(int32_t n_slices, const double* thickness) {
     SIMK_REQUIRE(n_slices >= 1 && thickness != nullptr, "a potential needs at least one slice");
     std::vector<double> dz(thickness, thickness + n_slices);
@@ -354,6 +363,7 @@ int simk_potential_read_transmission(simk_context* ctx, simk_potential* potentia
         SIMK_REQUIRE(slice >= 0 && slice < potential->impl.n_slices(), "slice out of range");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
         activate(ctx->impl);
+        refuse_capture(ctx->impl);
         prepare_transmissions(ctx->impl, potential->impl, energy);
         const long long N = potential->impl.g.count();
         download_complex(ctx->impl, potential->impl.t.as<float2>() + slice * N, N, re, im);
@@ -377,6 +387,7 @@ int simk_run(simk_context* ctx, simk_potential* potential, double energy, double
         }
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
         activate(ctx->impl);
+        refuse_capture(ctx->impl);
         run_waves(ctx->impl, potential->impl, energy, tilt_x, tilt_y, 1, in_re, in_im, pl, out_re, out_im);
     });
 }
@@ -391,6 +402,7 @@ int simk_run_batch(simk_context* ctx, simk_potential* potential, double energy, 
         SIMK_REQUIRE(std::isfinite(energy) && energy > 0, "the energy must be finite and positive");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
         activate(ctx->impl);
+        refuse_capture(ctx->impl);
         std::vector<int> pl{potential->impl.n_slices() - 1};
         run_waves(ctx->impl, potential->impl, energy, tilt_x, tilt_y, count, in_re, in_im, pl, out_re, out_im);
     });
@@ -445,6 +457,7 @@ int simk_apply_ctf(simk_context* ctx, const simk_grid* grid, double energy, cons
         SIMK_REQUIRE((out_re == nullptr) == (out_im == nullptr), "give both out_re and out_im, or neither");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
         activate(ctx->impl);
+        refuse_capture(ctx->impl);
         apply_ctf_device(ctx->impl, geom_of(grid), energy, *ctf, count, in_re, in_im, out_re, out_im, out_intensity);
     });
 }
@@ -563,6 +576,7 @@ int simk_build_probes(simk_context* ctx, const simk_grid* grid, const simk_probe
             SIMK_REQUIRE(std::isfinite(positions_xy[i]), "invalid position " + std::to_string(i / 2));
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
         activate(ctx->impl);
+        refuse_capture(ctx->impl);
         Context& c = ctx->impl;
         GridGeom g = geom_of(grid);
         const long long N = g.count();
@@ -670,6 +684,7 @@ int simk_scan_waves(simk_context* ctx, const simk_probe* probe, simk_potential* 
         SIMK_REQUIRE(potential->impl.ctx == &ctx->impl, "the potential belongs to another context");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
         activate(ctx->impl);
+        refuse_capture(ctx->impl);
         scan_waves(ctx->impl, *probe, potential->impl, n_positions, positions_xy, rows, columns, out_re, out_im);
     });
 }

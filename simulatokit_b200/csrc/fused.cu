@@ -1693,7 +1693,7 @@ int propagate_fused(Context& ctx, PotentialImpl& pot, double energy, double tx, 
     key_append(key, kspace_last);
     key_append(key, ctx.form);
     key_append(key, ctx.col_tile);
-      key_append(key, ctx.tma);
+    key_append(key, ctx.tma);
     key_append(key, ctx.tcgen05);
     key_append(key, ctx.composite);
     key_append(key, ctx.stream);

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <map>
@@ -38,6 +39,32 @@ inline void check_cuda(cudaError_t e, const char* what) {
 inline void copy_to_device(void* dst, const void* src, size_t bytes) {
     SIMK_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
     SIMK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+}
+
+// What a kernel's launches need and a device keeps for itself (function attributes hold for the device that was current, the
+// residency is its own): computed by the first launch on each device, whichever thread makes it. A static of the launch.
+class PerDevice {
+    static constexpr int kDevices = 64;
+    std::atomic<int> value_[kDevices] = {};  // 0: not computed, else the value + 1
+
+public:
+    // f() >= 0: sets the current device up and returns what its launches need to know. (Two threads may both call it.)
+    template <typename F> int get(F&& f) {
+        int device = 0;
+        SIMK_CUDA(cudaGetDevice(&device));
+        if (device >= kDevices) return f();
+        int v = value_[device].load(std::memory_order_acquire);
+        if (v == 0) {
+            v = f() + 1;
+            value_[device].store(v, std::memory_order_release);
+        }
+        return v - 1;
+    }
+};
+// The opt-in to `bytes` of dynamic shared memory, on the current device.
+template <typename K> int allow_shared(K kernel, size_t bytes) {
+    SIMK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return 0;
 }
 
 // ---- complex arithmetic on float2 / double2 -------------------------------------------------------------------------

@@ -277,12 +277,8 @@ void launch_t(const LinePlan& plan, void* data, long long nlines, int lines_per_
     int L = (int)std::max<size_t>(1, std::min<size_t>(16, budget / (2 * (size_t)lds * sizeof(V))));
     if (elem_stride == 1) L = std::min(L, 4);  // rows: a few whole lines per CTA
     const size_t smem = 2 * (size_t)L * lds * sizeof(V);
-    static bool attr_set[2] = {false, false};
-    const int which = sizeof(T) == 8 ? 1 : 0;
-    if (!attr_set[which]) {
-        SIMK_CUDA(cudaFuncSetAttribute(line_fft_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr_set[which] = true;
-    }
+    static PerDevice setup;
+    setup.get([] { return allow_shared(line_fft_kernel<T>, 200 * 1024); });
     SIMK_REQUIRE(smem <= 200 * 1024, "FFT line too long for one CTA");
     long long blocks = (nlines + L - 1) / L;
     SIMK_REQUIRE(blocks < (1LL << 31), "too many FFT lines");

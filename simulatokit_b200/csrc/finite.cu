@@ -31,7 +31,6 @@ namespace {
 constexpr double kKappaF = 0.0208865737082965;
 __constant__ double c_gl_x[kGaussNodes];
 __constant__ double c_gl_w[kGaussNodes];
-bool g_gl_ready[64] = {};
 }  // namespace
 
 // Gauss-Legendre nodes and weights on [-1, 1] by Newton's iteration on P_n (the classical Golub-Welsch-free method).
@@ -58,13 +57,15 @@ void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w) {
     }
 }
 
-void ensure_gauss_nodes(Context& ctx) {
-    if (g_gl_ready[ctx.device]) return;
-    std::vector<double> x, w;
-    gauss_legendre(kGaussNodes, x, w);
-    SIMK_CUDA(cudaMemcpyToSymbol(c_gl_x, x.data(), sizeof(double) * kGaussNodes));
-    SIMK_CUDA(cudaMemcpyToSymbol(c_gl_w, w.data(), sizeof(double) * kGaussNodes));
-    g_gl_ready[ctx.device] = true;
+void ensure_gauss_nodes(Context&) {
+    static PerDevice setup;
+    setup.get([] {
+        std::vector<double> x, w;
+        gauss_legendre(kGaussNodes, x, w);
+        SIMK_CUDA(cudaMemcpyToSymbol(c_gl_x, x.data(), sizeof(double) * kGaussNodes));
+        SIMK_CUDA(cudaMemcpyToSymbol(c_gl_w, w.data(), sizeof(double) * kGaussNodes));
+        return 0;
+    });
 }
 
 ElementAB element_ab(int z) {

@@ -1110,11 +1110,8 @@ void launch_rows_e(Context& ctx, const RegPlan& p, float2* psi, const float2* tm
     SIMK_REQUIRE(RB * p.T <= rows_threads(E), "row tile too large");
     const int lds = p.n + p.n / 16 + 1;
     const size_t smem = (size_t)RB * lds * sizeof(float2);
-    static bool set = false;
-    if (!set) {
-        SIMK_CUDA(cudaFuncSetAttribute(fused_rows_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-        set = true;
-    }
+    static PerDevice setup;
+    setup.get([] { return allow_shared(fused_rows_kernel<E>, 160 * 1024); });
     dim3 block(p.T, RB);
     const long long blocks = (nrows + RB - 1) / RB;
     fused_rows_kernel<E><<<(unsigned)blocks, block, smem, ctx.stream>>>(psi, tmul, p, nx, nrows, inv, fwd, scale,
@@ -1129,11 +1126,8 @@ void launch_cols_e(Context& ctx, const RegPlan& p, const ColArgs& a, int count) 
     while (TC > 1 && (TC * p.T > cols_threads(E) || a.ny % TC)) TC /= 2;
     SIMK_REQUIRE(TC * p.T <= cols_threads(E), "column tile too large");
     const size_t smem = (size_t)TC * p.n * sizeof(float2);
-    static bool set = false;
-    if (!set) {
-        SIMK_CUDA(cudaFuncSetAttribute(fused_cols_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-        set = true;
-    }
+    static PerDevice setup;
+    setup.get([] { return allow_shared(fused_cols_kernel<E>, 160 * 1024); });
     SIMK_REQUIRE(smem <= 160 * 1024, "column tile too large");
     dim3 block(TC, p.T);
     dim3 grid(a.ny / TC, count);
@@ -1148,11 +1142,8 @@ void launch_rows_ct(Context& ctx, const RegPlan& p, float2* psi, const float2* t
     constexpr int T = N / 8;
     constexpr int RB = (256 / T) > 0 ? (256 / T) : 1;
     const size_t smem = (size_t)RB * N * sizeof(float2);
-    static bool set = false;
-    if (!set) {
-        SIMK_CUDA(cudaFuncSetAttribute(fused_rows_ct<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-        set = true;
-    }
+    static PerDevice setup;
+    setup.get([] { return allow_shared(fused_rows_ct<N>, 160 * 1024); });
     SIMK_REQUIRE(nrows < (1LL << 31), "too many rows in one batch");
     dim3 block(T, RB);
     const long long blocks = (nrows + RB - 1) / RB;
@@ -1166,12 +1157,8 @@ template <int N, int TC, int MODE>
 void launch_cols_ct_m(Context& ctx, const RegPlan& p, const ColArgs& a, int count) {
     constexpr int T = N / 8;
     const size_t smem = (size_t)TC * N * sizeof(float2);
-    static bool set = false;
-    if (!set) {
-        SIMK_CUDA(cudaFuncSetAttribute(fused_cols_ct<N, TC, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       160 * 1024));
-        set = true;
-    }
+    static PerDevice setup;
+    setup.get([] { return allow_shared(fused_cols_ct<N, TC, MODE>, 160 * 1024); });
     dim3 block(TC, T);
     dim3 grid(a.ny / TC, count);
     fused_cols_ct<N, TC, MODE><<<grid, block, smem, ctx.stream>>>(a, p.tw);
@@ -1237,13 +1224,14 @@ bool launch_rows_tma_k(Context& ctx, const RegPlan& p, float2* psi, const float2
     if (nx % RB || nrows % RB || nrows >= (1LL << 31)) return false;
     const size_t smem = tma_pass_smem(N, RB, ENG);
     auto kern = fused_rows_tma<N, RB, ENG, IFW>;
-    static int occupancy = -1;
-    if (occupancy < 0) {
-        SIMK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    static PerDevice setup;
+    const int occupancy = setup.get([&] {
+        allow_shared(kern, 200 * 1024);
         SIMK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-        SIMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occupancy, kern, RB * T, smem));
-        occupancy = std::max(occupancy, fitting_blocks((const void*)kern, RB * T, smem, ctx.device));
-    }
+        int blocks = 0;
+        SIMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, RB * T, smem));
+        return std::max(blocks, fitting_blocks((const void*)kern, RB * T, smem, ctx.device));
+    });
     const int stack = ctx.tcgen05 == 2 ? 1 : 0;
     const int blocks_per_sm = pass_blocks_per_sm(occupancy, ENG, ENG == 3 ? tc5_blocks(N, RB) : 0, stack != 0);
     if (blocks_per_sm <= 0) return false;
@@ -1284,13 +1272,14 @@ bool launch_cols_tma_m(Context& ctx, const RegPlan& p, const ColArgs& a, int cou
     } else {
     const size_t smem = tma_pass_smem(N, TC, ENG);
     auto kern = fused_cols_tma<N, TC, MODE, ENG>;
-    static int occupancy = -1;
-    if (occupancy < 0) {
-        SIMK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    static PerDevice setup;
+    const int occupancy = setup.get([&] {
+        allow_shared(kern, 200 * 1024);
         SIMK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-        SIMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occupancy, kern, TC * T, smem));
-        occupancy = std::max(occupancy, fitting_blocks((const void*)kern, TC * T, smem, ctx.device));
-    }
+        int blocks = 0;
+        SIMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, TC * T, smem));
+        return std::max(blocks, fitting_blocks((const void*)kern, TC * T, smem, ctx.device));
+    });
     const int stack = ctx.tcgen05 == 2 ? 1 : 0;
     const int blocks_per_sm = pass_blocks_per_sm(occupancy, ENG, ENG == 3 ? tc5_blocks(N, TC) : 0, stack != 0);
     if (blocks_per_sm <= 0) return false;

@@ -161,12 +161,10 @@ __global__ void __launch_bounds__(LinePlanCfg<N, V>::NT_COLS, LinePlanCfg<N, V>:
 
 template <int N, bool BLUE, typename V> void launch_line(const LineArgs<V>& a, bool columns, cudaStream_t stream) {
     using P = LinePlanCfg<N, V>;
-    static bool set = false;
-    if (!set) {
-        SIMK_CUDA(cudaFuncSetAttribute(line_rows<N, BLUE, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM_ROWS));
-        SIMK_CUDA(cudaFuncSetAttribute(line_cols<N, BLUE, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM_COLS));
-        set = true;
-    }
+    static PerDevice setup;
+    setup.get([] {
+        return allow_shared(line_rows<N, BLUE, V>, P::SMEM_ROWS) + allow_shared(line_cols<N, BLUE, V>, P::SMEM_COLS);
+    });
     if (columns) {
         const long long blocks = a.lines / a.ny * ((a.ny + P::TC - 1) / P::TC);
         SIMK_REQUIRE(blocks < (1LL << 31), "too many FFT lines");

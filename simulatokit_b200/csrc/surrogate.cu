@@ -574,11 +574,8 @@ void fill_rows(const std::vector<int>& z, const std::vector<double>& rho, const 
 }
 
 void set_train_smem() {
-    static bool set = false;
-    if (!set) {
-        SIMK_CUDA(cudaFuncSetAttribute(k_sg_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrSmem));
-        set = true;
-    }
+    static PerDevice setup;
+    setup.get([] { return allow_shared(k_sg_train, kTrSmem); });
 }
 
 // Forward and backward of the doubled batch at (z, feats, target): the gradient into G (and, with lr > 0, the Adam step
@@ -605,12 +602,8 @@ double forward_backward(Context& ctx, float* P, float* G, const int* z, const fl
 }
 
 void set_infer_smem() {
-    static bool set = false;
-    if (!set) {
-        SIMK_CUDA(cudaFuncSetAttribute(k_sg_infer<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
-        SIMK_CUDA(cudaFuncSetAttribute(k_sg_infer<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
-        set = true;
-    }
+    static PerDevice setup;
+    setup.get([] { return allow_shared(k_sg_infer<true>, kTcSmem) + allow_shared(k_sg_infer<false>, kTcSmem); });
 }
 
 // Persistent grid: at most 4 blocks of 128 threads x 128 registers per SM, and no more warps than 16-query groups.

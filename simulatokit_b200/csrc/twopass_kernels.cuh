@@ -495,13 +495,13 @@ bool launch_two_rows(Context& ctx, const float2* table, float2* psi, const float
                      int fwd, float scale) {
     using P = RowPlan<N>;
     if (nrows >= (1LL << 31) - (1 << 20)) return false;
-    static int resident = -1;
-    if (resident < 0) {
-        SIMK_CUDA(cudaFuncSetAttribute(two_rows<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM));
+    static PerDevice setup;
+    const int resident = setup.get([] {
+        allow_shared(two_rows<N>, P::SMEM);
         int n = 0;
         SIMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, two_rows<N>, P::NT, P::SMEM));
-        resident = std::max(1, n);
-    }
+        return std::max(1, n);
+    });
     const long long tiles = (nrows + P::GR - 1) / P::GR, per = P::NT / P::GT;
     const int grid = (int)std::min<long long>((tiles + per - 1) / per, (long long)resident * ctx.sm_count);
     two_rows<N><<<grid, P::NT, P::SMEM, ctx.stream>>>(psi, tmul, table, (unsigned)nx, fast_div((unsigned)(nrows / nx)),
@@ -515,12 +515,8 @@ template <int N, int MODE> bool launch_two_cols_m(Context& ctx, const float2* ta
     using P = ColPlan<N>;
     const long long g = (a.ny + P::TC - 1) / P::TC, tiles = g * a.count;
     if (tiles >= (1LL << 31) - (1 << 20) || a.ny % 2) return false;  // rows of a multiple of 16 bytes
-    static bool set = false;
-    if (!set) {
-        SIMK_CUDA(cudaFuncSetAttribute(two_cols<N, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)P::smem(P::NB)));
-        set = true;
-    }
+    static PerDevice setup;
+    setup.get([] { return allow_shared(two_cols<N, MODE>, P::smem(P::NB)); });
     TwoDetect d{};
     if constexpr (MODE == 3) {
         const DetectorPlan::TileChannels& t = a.det->plan->tiles(P::TC);

@@ -850,7 +850,7 @@ int simk_surrogate_evaluate(simk_context* ctx, simk_surrogate* surrogate, int32_
         SIMK_REQUIRE(atomic_numbers && rho && zl && zu && out, "null argument");
         for (int i = 0; i < n; ++i)
             SIMK_REQUIRE(atomic_numbers[i] >= 1 && atomic_numbers[i] <= 103 && rho[i] > 0 &&
-                             infinite_in_reach(atomic_numbers[i], rho[i]),
+                             (rho[i] <= kInfiniteReach || infinite_in_reach(atomic_numbers[i], rho[i])),
                          "bad query");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
         activate(ctx->impl);

@@ -292,7 +292,6 @@ void finite_profiles_quadrature(Context& ctx, const FiniteDevice& d, long long n
 }
 
 bool infinite_in_reach(int z, double rho) {
-    if (rho <= 6000.0) return true;  // no B is above 990
     const ElementAB e = element_ab(z);
     return *std::max_element(e.B, e.B + 5) * rho <= 6000684.0;
 }

@@ -50,6 +50,7 @@ void infinite_points(Context& ctx, int n, const int* z_dev, const double* rho_de
 // Whether the radius is one of a full projection: finite, and B rho up to 6,000,684 for every term (all far past where it
 // underflows to 0; the Bessel functions of the C++ library end there, and such radii are refused).
 bool infinite_in_reach(int z, double rho);
+constexpr double kInfiniteReach = 6000.0;  // every element's reach is longer: no B is above 990
 std::vector<double> infinite_profiles(Context& ctx, const std::vector<int>& z, const std::vector<double>& rho);
 void finite_points(Context& ctx, const ElementAB* ab_dev, int n, const int* elem_dev, const double* rho_dev,
                    const double* zl_dev, const double* zu_dev, double* out_dev);

@@ -54,8 +54,6 @@ GridGeom geom_of(const simk_grid* g) {
     return r;
 }
 
-void activate(Context& c) { SIMK_CUDA(cudaSetDevice(c.device)); }
-
 // For calls that return waves to the host. They end in a wait, which a capture of the user's refuses, but by then what they
 // prepare (a potential's transmissions) has only been recorded, and the calls after it would take it for done.
 void refuse_capture(Context& c) {
@@ -106,12 +104,13 @@ int simk_context_create(int32_t device, simk_context** out) {
         try {
             SIMK_CUDA(cudaSetDevice(device));
             SIMK_CUDA(cudaStreamCreateWithFlags(&c->impl.own_stream, cudaStreamNonBlocking));
+            c->impl.stream = c->impl.own_stream;
+            device_context_made(c->impl);
         } catch (...) {
+            if (c->impl.own_stream) cudaStreamDestroy(c->impl.own_stream);
             delete c;
             throw;
         }
-        c->impl.stream = c->impl.own_stream;
-        device_context_made(device);
         *out = c;
     });
 }
@@ -123,9 +122,10 @@ int simk_context_destroy(simk_context* ctx) {
         cudaStreamSynchronize(ctx->impl.stream);
         cudaStream_t s = ctx->impl.own_stream;
         const int device = ctx->impl.device;
+        auto fence = std::move(ctx->impl.fence);
         delete ctx;
         if (s) cudaStreamDestroy(s);
-        device_context_gone(device);
+        device_context_gone(device, std::move(fence));
     });
 }
 
@@ -133,6 +133,7 @@ int simk_context_set_stream(simk_context* ctx, void* stream) {
     return guarded([&] {
         SIMK_REQUIRE(ctx, "context is null");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
+        device_stream_leaves(ctx->impl);
         ctx->impl.stream = stream ? static_cast<cudaStream_t>(stream) : ctx->impl.own_stream;
     });
 }
@@ -186,7 +187,7 @@ int simk_context_kernel_time(simk_context* ctx, const char* name, double* total_
     return guarded([&] {
         SIMK_REQUIRE(ctx && name && total_ms && launches && algorithmic_bytes, "null argument");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         SIMK_CUDA(cudaStreamSynchronize(ctx->impl.stream));
         ctx->impl.times.collect();
         auto it = ctx->impl.times.done.find(name);
@@ -238,7 +239,7 @@ int simk_context_synchronize(simk_context* ctx) {
     return guarded([&] {
         SIMK_REQUIRE(ctx, "context is null");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         SIMK_CUDA(cudaStreamSynchronize(ctx->impl.stream));
         check_device_error(ctx->impl);
     });
@@ -262,7 +263,7 @@ int simk_potential_from_atoms(simk_context* ctx, const simk_grid* grid, int32_t 
         SIMK_REQUIRE(n_atoms == 0 || (atomic_numbers && xyz && slice_of_atom), "null atom arrays");
         SIMK_REQUIRE(pi_choice == SIMK_PI_EXACT || pi_choice == SIMK_PI_ABTEM_FLOAT32, "unknown pi choice");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         auto p = std::make_unique<simk_potential>();
         p->impl.ctx = &ctx->impl;
         p->impl.g = geom_of(grid);
@@ -277,7 +278,7 @@ int simk_potential_from_values(simk_context* ctx, const simk_grid* grid, int32_t
     return guarded([&] {
         SIMK_REQUIRE(ctx && out && values, "null argument");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         auto p = std::make_unique<simk_potential>();
         p->impl.ctx = &ctx->impl;
         p->impl.g = geom_of(grid);
@@ -308,7 +309,7 @@ int simk_potential_read_slices(simk_context* ctx, simk_potential* potential, dou
     return guarded([&] {
         SIMK_REQUIRE(ctx && potential && values, "null argument");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         SIMK_CUDA(cudaStreamSynchronize(ctx->impl.stream));
         SIMK_CUDA(cudaMemcpy(values, potential->impl.V.ptr,
                              (size_t)potential->impl.n_slices() * potential->impl.g.count() * sizeof(double),
@@ -322,7 +323,7 @@ int simk_potential_tile(simk_context* ctx, const simk_potential* potential, int3
         SIMK_REQUIRE(ctx && potential && out, "null argument");
         SIMK_REQUIRE(potential->impl.ctx == &ctx->impl, "the potential belongs to another context");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         auto p = std::make_unique<simk_potential>();
         tile_potential(ctx->impl, potential->impl, repetitions_x, repetitions_y, repetitions_z, p->impl);
         SIMK_CUDA(cudaStreamSynchronize(ctx->impl.stream));
@@ -335,7 +336,7 @@ int simk_potential_project(simk_context* ctx, const simk_potential* potential, d
         SIMK_REQUIRE(ctx && potential && out, "null argument");
         SIMK_REQUIRE(potential->impl.ctx == &ctx->impl, "the potential belongs to another context");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         Context& c = ctx->impl;
         const long long N = potential->impl.g.count();
         DeviceBuffer d(N * sizeof(double));
@@ -362,7 +363,7 @@ int simk_potential_read_transmission(simk_context* ctx, simk_potential* potentia
         SIMK_REQUIRE(std::isfinite(energy) && energy > 0, "the energy must be finite and positive");
         SIMK_REQUIRE(slice >= 0 && slice < potential->impl.n_slices(), "slice out of range");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         refuse_capture(ctx->impl);
         prepare_transmissions(ctx->impl, potential->impl, energy);
         const long long N = potential->impl.g.count();
@@ -386,7 +387,7 @@ int simk_run(simk_context* ctx, simk_potential* potential, double energy, double
             SIMK_REQUIRE(q == 0 || pl[q] > pl[q - 1], "exit planes must be ascending and distinct");
         }
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         refuse_capture(ctx->impl);
         run_waves(ctx->impl, potential->impl, energy, tilt_x, tilt_y, 1, in_re, in_im, pl, out_re, out_im);
     });
@@ -401,7 +402,7 @@ int simk_run_batch(simk_context* ctx, simk_potential* potential, double energy, 
         SIMK_REQUIRE(in_re && in_im && out_re && out_im, "null argument");
         SIMK_REQUIRE(std::isfinite(energy) && energy > 0, "the energy must be finite and positive");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         refuse_capture(ctx->impl);
         std::vector<int> pl{potential->impl.n_slices() - 1};
         run_waves(ctx->impl, potential->impl, energy, tilt_x, tilt_y, count, in_re, in_im, pl, out_re, out_im);
@@ -413,7 +414,7 @@ int simk_probe_spectrum(simk_context* ctx, const simk_grid* grid, const simk_pro
     return guarded([&] {
         SIMK_REQUIRE(ctx && probe && re && im, "null argument");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         GridGeom g = geom_of(grid);
         DeviceBuffer f32, f64;
         probe_spectrum_device(ctx->impl, g, *probe, f32, &f64);
@@ -432,7 +433,7 @@ int simk_ctf_kernel(simk_context* ctx, const simk_grid* grid, double energy, con
     return guarded([&] {
         SIMK_REQUIRE(ctx && ctf && re && im, "null argument");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         GridGeom g = geom_of(grid);
         DeviceBuffer f64;
         ctf_kernel_device(ctx->impl, g, energy, *ctf, f64);
@@ -456,7 +457,7 @@ int simk_apply_ctf(simk_context* ctx, const simk_grid* grid, double energy, cons
         SIMK_REQUIRE(in_re && in_im, "null input");
         SIMK_REQUIRE((out_re == nullptr) == (out_im == nullptr), "give both out_re and out_im, or neither");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         refuse_capture(ctx->impl);
         apply_ctf_device(ctx->impl, geom_of(grid), energy, *ctf, count, in_re, in_im, out_re, out_im, out_intensity);
     });
@@ -470,7 +471,7 @@ int simk_gaussian_source_size_device(simk_context* ctx, int32_t nx, int32_t ny, 
     return guarded([&] {
         SIMK_REQUIRE(ctx && in_device && out_device, "null argument");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         gaussian_source_size_device(ctx->impl, nx, ny, value_count, sigma_x, sigma_y, sampling_x, sampling_y,
                                     in_device, out_device);
     });
@@ -483,7 +484,7 @@ int simk_gaussian_source_size(simk_context* ctx, int32_t nx, int32_t ny, int64_t
         SIMK_REQUIRE(nx >= 1 && ny >= 1 && value_count >= 1, "the scan needs at least one position and one value");
         SIMK_REQUIRE(value_count <= (1LL << 40) / ((long long)nx * ny), "the scan holds more than 2^40 values");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         Context& c = ctx->impl;
         const size_t bytes = (size_t)nx * ny * value_count * sizeof(double);
         DeviceBuffer d(bytes);
@@ -500,7 +501,7 @@ int simk_poisson_noise_device(simk_context* ctx, int64_t count, const double* in
     return guarded([&] {
         SIMK_REQUIRE(ctx && (count == 0 || (in_device && out_device)), "null argument");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         poisson_noise_device(ctx->impl, count, in_device, dose, samples, seed, out_device);
     });
 }
@@ -513,7 +514,7 @@ int simk_poisson_noise(simk_context* ctx, int64_t count, const double* in, doubl
         SIMK_REQUIRE(samples >= 1, "samples must be at least 1, got " + std::to_string(samples));
         SIMK_REQUIRE(count <= (1LL << 40) / samples, "more than 2^40 values and samples");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         Context& c = ctx->impl;
         if (count == 0) {
             poisson_noise_device(c, 0, nullptr, dose, samples, seed, nullptr);  // argument checks only
@@ -534,7 +535,7 @@ int simk_integrate_gradient_device(simk_context* ctx, int32_t nx, int32_t ny, do
     return guarded([&] {
         SIMK_REQUIRE(ctx && gx_device && gy_device && out_device, "null argument");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         integrate_gradient_device(ctx->impl, nx, ny, sampling_x, sampling_y, gx_device, gy_device, stride, out_device);
     });
 }
@@ -548,7 +549,7 @@ int simk_integrate_gradient(simk_context* ctx, int32_t nx, int32_t ny, double sa
         SIMK_REQUIRE(stride >= 1, "the component stride must be at least 1");
         SIMK_REQUIRE((long long)nx * ny <= (1LL << 28), "the gradient's images hold more than 2^28 pixels");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         Context& c = ctx->impl;
         const long long n = (long long)nx * ny;
         std::vector<double> h(2 * n);
@@ -575,7 +576,7 @@ int simk_build_probes(simk_context* ctx, const simk_grid* grid, const simk_probe
         for (int i = 0; i < 2 * count; ++i)
             SIMK_REQUIRE(std::isfinite(positions_xy[i]), "invalid position " + std::to_string(i / 2));
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         refuse_capture(ctx->impl);
         Context& c = ctx->impl;
         GridGeom g = geom_of(grid);
@@ -630,7 +631,7 @@ int simk_scan(simk_context* ctx, const simk_probe* probe, int32_t n_potentials, 
             SIMK_REQUIRE(std::isfinite(positions_xy[i]), "invalid position " + std::to_string(i / 2));
         auto pots = potentials_of(n_potentials, potentials);
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         Context& c = ctx->impl;
         const GridGeom& g = pots[0]->g;
         std::vector<long long> counts(n_detectors);
@@ -667,7 +668,7 @@ int simk_scan_device(simk_context* ctx, const simk_probe* probe, int32_t n_poten
                      "0 to 16 detectors");
         auto pots = potentials_of(n_potentials, potentials);
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         scan_device(ctx->impl, *probe, pots, n_positions, positions_xy_device, n_detectors, detectors, outputs_device);
     });
 }
@@ -683,7 +684,7 @@ int simk_scan_waves(simk_context* ctx, const simk_probe* probe, simk_potential* 
             SIMK_REQUIRE(std::isfinite(positions_xy[i]), "invalid position " + std::to_string(i / 2));
         SIMK_REQUIRE(potential->impl.ctx == &ctx->impl, "the potential belongs to another context");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         refuse_capture(ctx->impl);
         scan_waves(ctx->impl, *probe, potential->impl, n_positions, positions_xy, rows, columns, out_re, out_im);
     });
@@ -710,7 +711,7 @@ int simk_job_table_run(simk_context* ctx, int32_t n_jobs, const simk_job* jobs, 
             js[i].intensity = j.intensity;
         }
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         run_job_table(ctx->impl, js, done_ms);
     });
 }
@@ -722,7 +723,7 @@ int simk_fft2(simk_context* ctx, int32_t nx, int32_t ny, int32_t count, int32_t 
         SIMK_REQUIRE(nx >= 1 && ny >= 1 && count >= 1, "sizes must be positive");
         SIMK_REQUIRE(precision == 32 || precision == 64, "precision is 32 or 64");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         Context& c = ctx->impl;
         const long long N = (long long)nx * ny, total = N * count;
         const double scale = inverse ? 1.0 / (double)N : 1.0;
@@ -771,7 +772,7 @@ int simk_finite_profile(simk_context* ctx, int32_t n, const int32_t* atomic_numb
                          "rho must be positive and the limits finite");
         }
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         std::vector<int> z(atomic_numbers, atomic_numbers + n);
         std::vector<double> r(rho, rho + n), l(zl, zl + n), u(zu, zu + n);
         DeviceBuffer d(n * sizeof(double));
@@ -790,7 +791,7 @@ int simk_potential_from_atoms_finite(simk_context* ctx, const simk_grid* grid, i
         SIMK_REQUIRE(n_atoms >= 0 && (n_atoms == 0 || (atomic_numbers && xyz)), "null atom arrays");
         SIMK_REQUIRE(std::isfinite(error_bound) && error_bound > 0, "the error bound must be positive");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         auto p = std::make_unique<simk_potential>();
         p->impl.ctx = &ctx->impl;
         p->impl.g = geom_of(grid);
@@ -815,7 +816,7 @@ int simk_surrogate_train(simk_context* ctx, int32_t n_elements, const int32_t* a
                      "bad domain");
         SIMK_REQUIRE(n_samples <= (1LL << 27), "at most 2^27 training samples");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         std::vector<int> els(atomic_numbers, atomic_numbers + n_elements);
         auto s = std::make_unique<simk_surrogate>();
         s->impl = surrogate_train(ctx->impl, els, n_samples, steps, batch, learning_rate, seed, max_thickness, rho_min);
@@ -853,7 +854,7 @@ int simk_surrogate_evaluate(simk_context* ctx, simk_surrogate* surrogate, int32_
                              (rho[i] <= kInfiniteReach || infinite_in_reach(atomic_numbers[i], rho[i])),
                          "bad query");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         std::vector<int> z(atomic_numbers, atomic_numbers + n);
         std::vector<double> r(rho, rho + n), l(zl, zl + n), u(zu, zu + n);
         surrogate_evaluate(ctx->impl, *surrogate->impl, z, r, l, u, out);
@@ -864,7 +865,7 @@ int simk_surrogate_parameters(simk_context* ctx, simk_surrogate* surrogate, floa
     return guarded([&] {
         SIMK_REQUIRE(ctx && surrogate, "null argument");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         SurrogateImpl& s = *surrogate->impl;
         if (get) {
             SIMK_CUDA(cudaMemcpy(get, s.params.ptr, kSurrogateParams * sizeof(float), cudaMemcpyDeviceToHost));
@@ -892,7 +893,7 @@ int simk_surrogate_gradients(simk_context* ctx, simk_surrogate* surrogate, int32
         SIMK_REQUIRE(ctx && surrogate && n >= 1 && atomic_numbers && rho && zl && zu && target && gradients && loss,
                      "null argument");
         std::lock_guard<std::recursive_mutex> lk(ctx->impl.mu);
-        activate(ctx->impl);
+        const ActiveContext active(ctx->impl);
         std::vector<int> z(atomic_numbers, atomic_numbers + n);
         std::vector<double> r(rho, rho + n), l(zl, zl + n), u(zu, zu + n), t(target, target + n);
         *loss = surrogate_gradients(ctx->impl, *surrogate->impl, z, r, l, u, t, gradients);

@@ -97,8 +97,6 @@ template <typename V> __host__ __device__ __forceinline__ decltype(V::x) cabs2(V
 // Blocks come from and go back to the ones kept per device (hostio.cu).
 void* device_alloc(size_t n, size_t* got, int* device);
 void device_free(void* p, size_t bytes, int device);
-void device_context_made(int device);
-void device_context_gone(int device);
 
 struct DeviceBuffer {
     void* ptr = nullptr;

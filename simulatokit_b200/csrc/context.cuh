@@ -137,6 +137,7 @@ struct KernelTimes {
 };
 
 struct Context {
+    std::unique_ptr<StreamFence> fence;  // from device_context_made; outlives the buffers below
     int device = 0;
     int timing = 0;
     KernelTimes times;

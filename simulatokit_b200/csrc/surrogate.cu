@@ -691,8 +691,8 @@ std::unique_ptr<SurrogateImpl> surrogate_train(Context& ctx, const std::vector<i
     fill(OFF_W3, kHidden * kHidden, kHidden);
     fill(OFF_W4, kHidden, kHidden);
     copy_to_device(s->params.ptr, p.data(), kSurrogateParams * sizeof(float));
-    SIMK_CUDA(cudaMemset(s->m.ptr, 0, kSurrogateParams * sizeof(float)));
-    SIMK_CUDA(cudaMemset(s->v.ptr, 0, kSurrogateParams * sizeof(float)));
+    SIMK_CUDA(cudaMemsetAsync(s->m.ptr, 0, kSurrogateParams * sizeof(float), ctx.stream));
+    SIMK_CUDA(cudaMemsetAsync(s->v.ptr, 0, kSurrogateParams * sizeof(float), ctx.stream));
     // the training set, labelled F = P / P_inf with P by the float64 device quadrature
     const long long n = n_samples;
     std::vector<int> all_z(n);

@@ -1,14 +1,26 @@
-// A CUDA runtime without a GPU for CPU tests of host code: devices, function attributes and launches are only recorded.
+// A CUDA runtime without a GPU for CPU tests of host code: devices, function attributes, launches and the order that events
+// give to streams are only recorded. A stream is a count of the work queued on it; an event holds the counts that have to
+// be reached before it, and a host that waits for it knows that they are. Nothing else tells the host: cudaFree and
+// cudaDeviceSynchronize do not wait here.
 #include <cuda_runtime_api.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <map>
 #include <utility>
 
 namespace {
-int device = 0, launches = 0, refused = 0;
+int device = 0, launches = 0, refused = 0, unordered_frees = 0, recorded_in_capture = 0, blocks = 0;
 size_t config_shared = 0;
 std::map<std::pair<int, const void*>, int> shared_allowed, times_allowed;
+using Order = std::map<void*, long>;  // per stream, how much of its work comes before
+std::map<void*, Order> streams, events;
+Order host;  // what the host has seen finished
+std::map<void*, bool> capturing;
+template <typename H> H made() { return static_cast<H>(static_cast<void*>(std::malloc(16))); }
+void later(Order& a, const Order& b) {
+    for (auto& kv : b) a[kv.first] = std::max(a[kv.first], kv.second);
+}
 }  // namespace
 
 extern "C" {
@@ -19,6 +31,83 @@ int fake_most_opt_ins() {
     int most = 0;
     for (auto& kv : times_allowed) most = std::max(most, kv.second);
     return most;
+}
+// Queues work on a stream (or has a capture record it); blocks given back to a pool while work was queued on some stream
+// that the host had not seen finished; events recorded on a stream that a capture had; blocks handed out and not given
+// back.
+void fake_work(cudaStream_t s) { streams[s][s] += !capturing[s]; }
+void fake_capture(cudaStream_t s, int on) { capturing[s] = on != 0; }
+int fake_unordered_frees() { return unordered_frees; }
+int fake_recorded_in_capture() { return recorded_in_capture; }
+int fake_blocks() { return blocks; }
+
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
+    *s = made<cudaStream_t>();
+    streams[*s][*s] = 0;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
+cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* status) {
+    *status = capturing[s] ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode*) { return cudaSuccess; }
+cudaError_t cudaStreamQuery(cudaStream_t s) { return streams[s][s] > host[s] ? cudaErrorNotReady : cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+    *e = made<cudaEvent_t>();
+    return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    if (capturing[s]) ++recorded_in_capture;
+    events[e] = streams[s];
+    return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+    later(host, events[e]);
+    return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+    events.erase(e);
+    return cudaSuccess;
+}
+cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps*) {
+    *p = made<cudaMemPool_t>();
+    return cudaSuccess;
+}
+cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { return cudaSuccess; }
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
+cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, cudaMemPoolAttr, void* v) {
+    *static_cast<unsigned long long*>(v) = 0;
+    return cudaSuccess;
+}
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
+cudaError_t cudaMallocFromPoolAsync(void** p, size_t, cudaMemPool_t, cudaStream_t) {
+    *p = made<void*>();
+    ++blocks;
+    return cudaSuccess;
+}
+cudaError_t cudaFreeAsync(void*, cudaStream_t) {
+    --blocks;
+    unordered_frees += std::any_of(streams.begin(), streams.end(), [](auto& s) { return s.second[s.first] > host[s.first]; });
+    return cudaSuccess;
+}
+cudaError_t cudaMalloc(void** p, size_t) {
+    *p = made<void*>();
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void*) { return cudaSuccess; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+    *p = std::malloc(n);
+    return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void* p) {
+    std::free(p);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void*, const void*, size_t, cudaMemcpyKind, cudaStream_t s) {
+    fake_work(s);
+    return cudaSuccess;
 }
 
 cudaError_t cudaGetDevice(int* d) {

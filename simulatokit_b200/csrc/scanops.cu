@@ -257,8 +257,9 @@ __device__ double poisson_draw(double lambda, Xoshiro& g, int* err) {
 constexpr int kPoissonTile = 2048;
 constexpr int kPoissonBins = 12;  // 0: nothing to draw; 1 + whole part of a mean below 10; 11: PTRS
 
-__global__ void __launch_bounds__(256) k_poisson(const double* __restrict__ in, double* __restrict__ out, long long count,
-                                                 int samples, double dose, uint64_t seed, int* err) {
+// `out` may be `in` where samples is 1: a tile is read whole before it is written.
+__global__ void __launch_bounds__(256) k_poisson(const double* in, double* out, long long count, int samples, double dose,
+                                                 uint64_t seed, int* err) {
     __shared__ double mean[kPoissonTile];  // then the draws
     __shared__ unsigned short order[kPoissonTile];
     __shared__ int fill[kPoissonBins];
@@ -322,8 +323,8 @@ __global__ void __launch_bounds__(256) k_poisson(const double* __restrict__ in, 
 // The reference's own stream (ScanOperations.swift:80-117): one generator seeded by `seed`, every sample's values drawn
 // in order, so that a seed gives the reference's draws. The number of uniforms a draw takes depends on the draws, so
 // the chain cannot be split: one thread walks it. err bits as k_poisson.
-__global__ void k_poisson_sequential(const double* __restrict__ in, double* __restrict__ out, long long count,
-                                     int samples, double dose, uint64_t seed, int* err) {
+__global__ void k_poisson_sequential(const double* in, double* out, long long count, int samples, double dose,
+                                     uint64_t seed, int* err) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     Xoshiro g;
     seed_xoshiro(g, seed);
@@ -509,8 +510,8 @@ void poisson_noise_device(Context& ctx, long long count, const double* in, doubl
         if (ctx.poisson_stream == 1)
             k_poisson_sequential<<<1, 1, 0, ctx.stream>>>(in, out, count, samples, dose, seed, ctx.post_flag.as<int>());
         else
-            k_poisson<<<(int)std::min<long long>((count + kPoissonTile - 1) / kPoissonTile * samples, 148LL * 16), 256, 0,
-                        ctx.stream>>>(in, out, count, samples, dose, seed, ctx.post_flag.as<int>());
+            k_poisson<<<(int)std::min<long long>((count + kPoissonTile - 1) / kPoissonTile * samples, 16LL * ctx.sm_count),
+                        256, 0, ctx.stream>>>(in, out, count, samples, dose, seed, ctx.post_flag.as<int>());
     }
     ++ctx.launches;
     SIMK_CUDA(cudaGetLastError());

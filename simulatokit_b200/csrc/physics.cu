@@ -337,7 +337,7 @@ void build_potential_from_atoms(Context& ctx, PotentialImpl& pot, int pi_choice,
     };
     auto accumulate = [&](int slices, const int* ptr, int first0, int more) {
         const int across = std::min(slices, 65535);
-        k_accum_spectra<<<dim3(std::max(1, std::min(blocks_for(N), 148 * 16 / across + 1)), across), 256, 0, ctx.stream>>>(
+        k_accum_spectra<<<dim3(std::max(1, std::min(blocks_for(N), 16 * ctx.sm_count / across + 1)), across), 256, 0, ctx.stream>>>(
             spec.as<double2>(), delta.as<double2>(), kern.as<double>(), elem_of, ptr, slices, first0, more, N);
         ++ctx.launches;
     };

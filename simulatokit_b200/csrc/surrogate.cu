@@ -773,12 +773,18 @@ std::unique_ptr<SurrogateImpl> surrogate_train(Context& ctx, const std::vector<i
     return s;
 }
 
+constexpr size_t kKeptQueries = 64u << 20;  // 1.5 million queries
 void surrogate_evaluate(Context& ctx, const SurrogateImpl& s, const std::vector<int>& z, const std::vector<double>& rho,
                         const std::vector<double>& zl, const std::vector<double>& zu, double* out_host) {
     const int n = (int)z.size();
     if (n == 0) return;
     set_infer_smem();
-    // one buffer kept in the context: rho, zl, zu, the full projections, the results, the atomic numbers
+    // one buffer kept in the context, up to kKeptQueries bytes of it: rho, zl, zu, the full projections, the results, the
+    // atomic numbers
+    struct Bound {
+        DeviceBuffer& kept;
+        ~Bound() { if (kept.bytes > kKeptQueries) kept.release(); }
+    } bound{ctx.evaluate_work};
     ctx.evaluate_work.ensure((size_t)n * (5 * sizeof(double) + sizeof(int)));
     double* const dr = ctx.evaluate_work.as<double>();
     double *const dl = dr + n, *const du = dl + n, *const dp = du + n, *const dout = dp + n;

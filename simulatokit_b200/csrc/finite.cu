@@ -64,6 +64,7 @@ void ensure_gauss_nodes(Context&) {
         gauss_legendre(kGaussNodes, x, w);
         SIMK_CUDA(cudaMemcpyToSymbol(c_gl_x, x.data(), sizeof(double) * kGaussNodes));
         SIMK_CUDA(cudaMemcpyToSymbol(c_gl_w, w.data(), sizeof(double) * kGaussNodes));
+        SIMK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // there before a non-blocking stream reads them
         return 0;
     });
 }

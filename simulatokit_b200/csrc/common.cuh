@@ -97,6 +97,9 @@ template <typename V> __host__ __device__ __forceinline__ decltype(V::x) cabs2(V
 // Blocks come from and go back to the ones kept per device (hostio.cu).
 void* device_alloc(size_t n, size_t* got, int* device);
 void device_free(void* p, size_t bytes, int device);
+// What the device's pool holds beyond the blocks in use: free for further blocks, but not counted by
+// cudaMemGetInfo.
+size_t device_held_free(int device);
 
 struct DeviceBuffer {
     void* ptr = nullptr;

@@ -1836,6 +1836,7 @@ Context::Tuned autotune(Context& ctx, PotentialImpl& pot, double energy, double 
     const long long N = g.count();
     size_t free_b = 0, total_b = 0;
     SIMK_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    free_b += device_held_free(ctx.device);
     long long cap = (long long)(free_b / 2 / (2 * (size_t)N * sizeof(float2)));
     cap = std::max(1LL, std::min(cap, 1024LL));  // per grid, not per call: the caller's batches cap themselves
     (void)max_waves;

@@ -149,6 +149,14 @@ void device_free(void* p, size_t bytes, int device) {
     if (current != device) cudaSetDevice(current);
 }
 
+size_t device_held_free(int device) {
+    std::lock_guard<std::mutex> lk(g_pools_mutex);
+    DevicePool& d = device_pool(device);
+    unsigned long long held = 0;
+    if (!d.pool || cudaMemPoolGetAttribute(d.pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess) return 0;
+    return held > d.live ? (size_t)held - d.live : 0;
+}
+
 void device_context_made(Context& ctx) {
     auto fence = std::make_unique<StreamFence>();
     fence->event = make_event();

@@ -12,6 +12,7 @@
 namespace {
 int device = 0, launches = 0, refused = 0, unordered_frees = 0, recorded_in_capture = 0, blocks = 0;
 size_t config_shared = 0;
+unsigned long long reserved = 0;
 std::map<std::pair<int, const void*>, int> shared_allowed, times_allowed;
 using Order = std::map<void*, long>;  // per stream, how much of its work comes before
 std::map<void*, Order> streams, events;
@@ -40,6 +41,7 @@ void fake_capture(cudaStream_t s, int on) { capturing[s] = on != 0; }
 int fake_unordered_frees() { return unordered_frees; }
 int fake_recorded_in_capture() { return recorded_in_capture; }
 int fake_blocks() { return blocks; }
+void fake_reserve(unsigned long long n) { reserved = n; }  // what every pool holds
 
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
     *s = made<cudaStream_t>();
@@ -78,7 +80,7 @@ cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps*) {
 cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { return cudaSuccess; }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
 cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, cudaMemPoolAttr, void* v) {
-    *static_cast<unsigned long long*>(v) = 0;
+    *static_cast<unsigned long long*>(v) = reserved;
     return cudaSuccess;
 }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }

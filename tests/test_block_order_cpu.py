@@ -25,6 +25,7 @@ void fake_capture(cudaStream_t, int);
 int fake_unordered_frees();
 int fake_recorded_in_capture();
 int fake_blocks();
+void fake_reserve(unsigned long long);
 }
 using namespace simk;
 
@@ -103,6 +104,9 @@ int main() {
     DeviceBuffer last(8);
     last.release();
     say("one-gone");
+    DeviceBuffer some(1 << 20);
+    fake_reserve(3 << 20);
+    printf("held %zu\n", device_held_free(0));
 }
 """
 
@@ -124,7 +128,8 @@ def test_blocks_go_back_behind_every_stream(tmp_path):
                   exe], [exe]):
         r = subprocess.run(args, capture_output=True, text=True)
         assert r.returncode == 0, r.stdout + r.stderr
-    lines = [line.split() for line in r.stdout.splitlines()]
+    *lines, held = [line.split() for line in r.stdout.splitlines()]
+    assert held == ["held", str(2 << 20)]  # of what the pool holds, the block in use is not free
     assert [line[0] for line in lines] == ["in-call", "after-call", "other-context", "stream-changed", "captured", "nested",
                                            "one-gone"]
     for what, unordered, recorded_in_capture, blocks in lines:

@@ -215,7 +215,7 @@ template <int DIR> __device__ __forceinline__ void pbfly8(double2 (&v)[8]) { bfl
 // The first factor A of the step R = A B.
 constexpr int dft_first(int r) {
     return r == 6 ? 2 : r == 10 ? 2 : r == 12 ? 3 : r == 15 ? 3 : r == 16 ? 4 : r == 18 ? 3 : r == 20 ? 4 : r == 24 ? 3
-           : r == 25 ? 5 : r == 30 ? 5 : r == 32 ? 4 : r == 40 ? 5 : 0;
+           : r == 25 ? 5 : r == 30 ? 5 : r == 32 ? 4 : 0;
 }
 
 // X[k1 + A k2] = sum_n2 W_R^{n2 k1} W_B^{n2 k2} sum_n1 x[B n1 + n2] W_A^{n1 k1}

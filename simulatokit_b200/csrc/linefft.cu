@@ -13,7 +13,6 @@ namespace simk {
 #define SIMK_BLUE(n)                                                                             \
     extern template void launch_line<n, true, float2>(const LineArgs<float2>&, bool, cudaStream_t);     \
     extern template void launch_line<n, true, double2>(const LineArgs<double2>&, bool, cudaStream_t);
-SIMK_BLUE(128)
 SIMK_BLUE(256)
 SIMK_BLUE(512)
 SIMK_BLUE(1024)
@@ -76,12 +75,11 @@ std::vector<float2> line_table(int n, int r1, double scale) {
     return t;
 }
 
-bool line_bluestein_length(int N) { return N == 128 || N == 256 || N == 512 || N == 1024; }
+bool line_bluestein_length(int N) { return N == 256 || N == 512 || N == 1024; }
 
 template <typename V> void launch_line_any(int N, bool blue, const LineArgs<V>& a, bool columns, cudaStream_t stream) {
     if (blue) {
         switch (N) {
-            case 128: launch_line<128, true, V>(a, columns, stream); return;
             case 256: launch_line<256, true, V>(a, columns, stream); return;
             case 512: launch_line<512, true, V>(a, columns, stream); return;
             default: launch_line<1024, true, V>(a, columns, stream); return;

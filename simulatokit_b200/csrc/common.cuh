@@ -41,8 +41,9 @@ inline void copy_to_device(void* dst, const void* src, size_t bytes) {
     SIMK_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
 }
 
-// What a kernel's launches need and a device keeps for itself (function attributes hold for the device that was current, the
-// residency is its own): computed by the first launch on each device, whichever thread makes it. A static of the launch.
+// What a kernel's launches need and a device keeps for itself (function attributes hold for the device that was
+// current, the residency is its own): computed by the first launch on each device, whichever thread makes it. A static
+// of the launch.
 class PerDevice {
     static constexpr int kDevices = 64;
     std::atomic<int> value_[kDevices] = {};  // 0: not computed, else the value + 1

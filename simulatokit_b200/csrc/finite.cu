@@ -187,7 +187,8 @@ __device__ double infinite_profile_dev(const ElementAB& e, double rho) {
 }
 
 // The full projections at n (atomic number, radius) points, one thread each: 125 exponentials in place of the same sum
-// by the host's Bessel functions, 2.7 us a point there (an evaluation of 100,000 points with a 4,096-sample gradient: 287 -> 1.9 ms).
+// by the host's Bessel functions, 2.7 us a point there (an evaluation of 100,000 points with a 4,096-sample gradient:
+// 287 -> 1.9 ms).
 __global__ void k_infinite_points(const int* __restrict__ z, const double* __restrict__ rho, int n,
                                   const ElementAB* __restrict__ elements, double* __restrict__ out) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)

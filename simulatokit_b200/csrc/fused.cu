@@ -611,7 +611,8 @@ constexpr int tc_min_blocks(int threads, int eng) {
 }
 
 template <int N, int TC, int MODE, int ENG>
-__global__ void __launch_bounds__(TC * (N / 8), tc_min_blocks(TC * (N / 8), ENG)) fused_cols_tma(const __grid_constant__ CUtensorMap map,
+__global__ void __launch_bounds__(TC * (N / 8), tc_min_blocks(TC * (N / 8), ENG))
+    fused_cols_tma(const __grid_constant__ CUtensorMap map,
                                                                const __grid_constant__ CUtensorMap pmap,
                                                                float2* __restrict__ psi, float pscale, int ny,
                                                                int count, const float2* __restrict__ tw, int* err,

@@ -54,7 +54,7 @@ struct HostStage {
 
 // dst[i] = (re[i], im[i]) rounded to float32, stream-ordered; the host arrays may be reused when it returns.
 void upload_complex(Context& ctx, float2* dst, const double* re, const double* im, long long n);
-// re[i], im[i] = src[i] (either may be null), and intensity[i] = re^2 + im^2 where it is not null. Returns when the host
+// re[i], im[i] = src[i] (both null: not wanted), and intensity[i] = re^2 + im^2 where it is not null. Returns when the host
 // arrays are written (the stream has then reached this point).
 void download_complex(Context& ctx, const float2* src, long long n, double* re, double* im, double* intensity = nullptr);
 

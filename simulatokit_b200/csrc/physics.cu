@@ -337,7 +337,8 @@ void build_potential_from_atoms(Context& ctx, PotentialImpl& pot, int pi_choice,
     };
     auto accumulate = [&](int slices, const int* ptr, int first0, int more) {
         const int across = std::min(slices, 65535);
-        k_accum_spectra<<<dim3(std::max(1, std::min(blocks_for(N), 16 * ctx.sm_count / across + 1)), across), 256, 0, ctx.stream>>>(
+        const int blocks = std::max(1, std::min(blocks_for(N), 16 * ctx.sm_count / across + 1));
+        k_accum_spectra<<<dim3(blocks, across), 256, 0, ctx.stream>>>(
             spec.as<double2>(), delta.as<double2>(), kern.as<double>(), elem_of, ptr, slices, first0, more, N);
         ++ctx.launches;
     };
@@ -582,7 +583,8 @@ __device__ __forceinline__ double block_sum(double s) {
 }
 __global__ void __launch_bounds__(256) k_norm2_shares(const double2* a, long long N, double* out) {
     double s = 0.0;
-    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < N; i += kNormBlocks * 256LL) s += a[i].x * a[i].x + a[i].y * a[i].y;
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < N; i += kNormBlocks * 256LL)
+        s += a[i].x * a[i].x + a[i].y * a[i].y;
     s = block_sum(s);
     if (threadIdx.x == 0) out[1 + blockIdx.x] = s;
 }

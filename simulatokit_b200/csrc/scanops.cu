@@ -249,11 +249,12 @@ __device__ double poisson_draw(double lambda, Xoshiro& g, int* err) {
 // the mix of a frozen-phonon configuration's seed (FrozenPhonons.swift:122-130). err bit 2: a value times the dose is
 // not finite (the reference's sampler would never return); its draws are then 0.
 //
-// Bound by the integer and FP64 work of the draws, and by divergence: a draw takes about mean + 1 products below a mean of
-// 10 and the PTRS arithmetic above, and a warp takes as long as its longest lane on each. A block therefore takes
+// Bound by the integer and FP64 work of the draws, and by divergence: a draw takes about mean + 1 products below a mean
+// of 10 and the PTRS arithmetic above, and a warp takes as long as its longest lane on each. A block therefore takes
 // kPoissonTile values at a time and draws them in the order of their means (a counting sort on the whole part of the
 // mean, in shared memory), so that a warp's lanes take alike; each value has its own generator, so the order changes
-// nothing. Means of 0 are done by then. 4.2 M values of means 0 to 20 (three quarters below 4): 126 -> 107 us, at 70 % of the issue slots (the generators' 64-bit integer work).
+// nothing. Means of 0 are done by then. 4.2 M values of means 0 to 20 (three quarters below 4): 126 -> 107 us, at 70 %
+// of the issue slots (the generators' 64-bit integer work).
 constexpr int kPoissonTile = 2048;
 constexpr int kPoissonBins = 12;  // 0: nothing to draw; 1 + whole part of a mean below 10; 11: PTRS
 
@@ -474,8 +475,8 @@ void gaussian_source_size_device(Context& ctx, int nx, int ny, long long v, doub
                 SIMK_REQUIRE(tiles < (1LL << 31), "the scan's values are too many for one filter launch");
                 const size_t smem = 2 * (size_t)(rows + 2 * kQ) * 32 * sizeof(double);  // two staging buffers
                 int per_sm = 0;
-                // a warp for every kQ outputs of a tile: short axes leave fewer idle and more blocks on an SM (axes of 32 with
-                // 4 M values: 34.1 us a pass with 256 threads, 30.5 with 128)
+                // a warp for every kQ outputs of a tile: short axes leave fewer idle and more blocks on an SM (axes of
+                // 32 with 4 M values: 34.1 us a pass with 256 threads, 30.5 with 128)
                 const int threads = std::max(128, std::min(256, 32 * ((KT + kQ - 1) / kQ)));
                 SIMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gauss_axis_tiled, threads, smem));
                 const long long resident = (long long)ctx.sm_count * std::max(1, per_sm);

@@ -227,11 +227,12 @@ __device__ __forceinline__ void tc5_read(const Tc5& c, uint32_t taddr, float (&d
     }
 }
 
-// The stages' twiddles of this thread's vector (its mapping as in tc5_fft), kept in registers: read from the table inside
-// the stages, their latency stood in every tile's way (long scoreboard 2.1 of 8 stall cycles an instruction). 512^2 x 256 waves,
-// with the row passes instantiated per (inverse, forward): rows 698 -> 576 us, columns 548 -> 503; 256^2 153 -> 141, 126 ->
-// 121.
-template <int N, int LINES, bool COLS> __device__ __forceinline__ void tc5_twiddles(Tc5& c, const float2* __restrict__ tw, int tid) {
+// The stages' twiddles of this thread's vector (its mapping as in tc5_fft), kept in registers: read from the table
+// inside the stages, their latency stood in every tile's way (long scoreboard 2.1 of 8 stall cycles an instruction).
+// 512^2 x 256 waves, with the row passes instantiated per (inverse, forward): rows 698 -> 576 us, columns 548 -> 503;
+// 256^2 153 -> 141, 126 -> 121.
+template <int N, int LINES, bool COLS>
+__device__ __forceinline__ void tc5_twiddles(Tc5& c, const float2* __restrict__ tw, int tid) {
     constexpr int R = N / 256, NV = N / 16, NSA = R;
     const int warp = tid >> 5, lane = tid & 31;
     const int h = (warp >> 2) & 1, v = (warp >> 3) * 128 + (warp & 3) * 32 + lane;

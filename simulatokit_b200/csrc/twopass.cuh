@@ -24,13 +24,14 @@ constexpr int kTwoColsAbove = 128;
 
 // Whether lines of n points have a plan here.
 bool twopass_length(int n);
-// The plan's twiddle table of n divided by `points` (the inverse transform's 1 / (nx ny) in the columns' way back), created
-// on first use (allocates and copies: not inside a stream capture).
+// The plan's twiddle table of n divided by `points` (the inverse transform's 1 / (nx ny) in the columns' way back),
+// created on first use (allocates and copies: not inside a stream capture).
 const float2* twopass_table(Context& ctx, int n, long long points = 1);
 // The row pass over nrows = count nx rows of ny points: [inverse], x t x scale, [forward]. False: no plan for ny.
 bool twopass_rows(Context& ctx, float2* psi, const float2* tmul, int nx, int ny, long long nrows, int inv, int fwd,
                   float scale);
-// The column pass over lines of nx > kTwoColsAbove points (false otherwise, or without a plan); with mode 3 *groups receives the column groups of the partial sums.
+// The column pass over lines of nx > kTwoColsAbove points (false otherwise, or without a plan); with mode 3 *groups
+// receives the column groups of the partial sums.
 bool twopass_cols(Context& ctx, int nx, const TwoPassCols& a, int* groups);
 
 }  // namespace simk

@@ -26,13 +26,6 @@ template <int N> struct TwoPlan { static constexpr int R1 = 0, R2 = 0; };
 #include "twopass_plans.inc"
 #undef SIMK_TWO_PLAN
 
-// The same pointer, unknown to the compiler: the addresses that a line's loads and stores share are computed again for
-// the stores instead of being kept in registers (spilled) through the transforms.
-template <typename T> __device__ __forceinline__ T* again(T* p) {
-    asm volatile("" : "+l"(p));
-    return p;
-}
-
 template <int GT> __device__ __forceinline__ void group_sync(int id) {
     if constexpr (GT == 32) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(GT) : "memory");
@@ -64,7 +57,8 @@ template <int N> struct RowPlan {
     static constexpr int NT = WARP ? 128 : GT;
     static constexpr int LD = R1 | 1;  // odd: column walks of M touch every bank pair
     static constexpr int QA = (GR * R2 + GT - 1) / GT, QB = (GR * R1 + GT - 1) / GT;
-    static constexpr int BLOCKS = (R2 <= 16 ? 768 : R2 <= 25 ? 640 : 512) / NT;  // an SM, asked of the compiler: 85, 102 or 128 registers
+    // an SM, asked of the compiler: 85, 102 or 128 registers
+    static constexpr int BLOCKS = (R2 <= 16 ? 768 : R2 <= 25 ? 640 : 512) / NT;
     static constexpr size_t SMEM = (size_t)(N + NT / GT * GR * R2 * LD) * sizeof(float2);
 };
 
@@ -201,9 +195,10 @@ __global__ void __launch_bounds__(RowPlan<N>::NT, RowPlan<N>::BLOCKS)
 // and belongs to sub-block i % SUBS. TMA brings a tile in and takes it out; the load of tile i + NB is issued by the
 // sub-block that had tile i, once the store of tile i has read its buffer (asked for in the middle of its next tile).
 // Bound at 512 by the latency of a tile's three steps at four warps a scheduler (512 waves: 505 us between two slices,
-// 4.25 TB/s; 437 us the mean of a 6-slice scan's launches, as the times below; FMA pipe and issue near half busy). Tiles loaded and stored from registers instead, without TMA: 541 us, most of it
-// the loads' latency; tiles of 16 columns that way 550 us; P's first values asked for in step B 482 us, before the
-// tile's wait 440 us. Programmatic dependent launch of the passes cost 4 % at 512^2 (5 % at 256^2) and is not used.
+// 4.25 TB/s; 437 us the mean of a 6-slice scan's launches, as the times below; FMA pipe and issue near half busy).
+// Tiles loaded and stored from registers instead, without TMA: 541 us, most of it the loads' latency; tiles of 16
+// columns that way 550 us; P's first values asked for in step B 482 us, before the tile's wait 440 us. Programmatic
+// dependent launch of the passes cost 4 % at 512^2 (5 % at 256^2) and is not used.
 // All three steps work in place: step A's value (j, k) lies in the row j + R2 k that item j owns, with the rows of
 // j and j ^ 1 exchanged for odd k where R2 is even, so that two neighbouring items always lie in different halves of the
 // 128 bytes that a half-warp reads at once, along j as along k (items j and j ^ 1 are in one warp).
@@ -281,7 +276,10 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
         b = w + (r - g * (whole ? subs : order.rest.d));
     };
     const unsigned first = blockIdx.x * subs;
-    auto tile_of = [&](unsigned i) { const unsigned q = i / order.subs; return first + q * round + (i - q * subs); };  // the block's i-th tile
+    auto tile_of = [&](unsigned i) {  // the block's i-th tile
+        const unsigned q = i / order.subs;
+        return first + q * round + (i - q * subs);
+    };
     auto issue = [&](unsigned i) {
         const unsigned tile = tile_of(i);
         if (tile >= ntiles) return;
@@ -545,8 +543,8 @@ template <int N, int MODE> bool launch_two_cols_m(Context& ctx, const float2* ta
     const float2* const back = MODE == 0 ? twopass_table(ctx, N, (long long)N * a.ny) : table;
     const CUtensorMap map = encode_tensor_map_2d(a.psi, 2ULL * a.ny, (unsigned long long)a.count * N, 2 * P::TC, P::BOXH);
     two_cols<N, MODE><<<grid, P::NT * subs, P::smem(buffers), ctx.stream>>>(
-        map, a.psi, MODE == 2 ? a.spectrum : a.P, table, back, scale, (float)(inverse - (double)scale), a.ny, order, buffers,
-        ctx.err_flag.as<int>(), a.p_row, a.rx, a.ry, d);
+        map, a.psi, MODE == 2 ? a.spectrum : a.P, table, back, scale, (float)(inverse - (double)scale), a.ny, order,
+        buffers, ctx.err_flag.as<int>(), a.p_row, a.rx, a.ry, d);
     SIMK_CUDA(cudaGetLastError());
     ++ctx.launches;
     return true;

@@ -49,10 +49,11 @@ __device__ __forceinline__ unsigned operator/(unsigned n, const FastDiv& f) {
 // and the FMA pipe elsewhere (500 = 20 x 25: 3.5 TB/s, 166 us for 144 waves, FMA pipe near half busy).
 // A group of GT threads takes GR rows at a time: one warp where R1 and R2 divide its lanes evenly (256, 512, 1024 and
 // 128 points: no barrier beyond __syncwarp), else a block.
-template <int N> struct RowPlan {
+// SPREAD: at 512 a warp takes one row instead of two, half of step B's lanes idle, for launches of few rows.
+template <int N, bool SPREAD = false> struct RowPlan {
     static constexpr int R1 = TwoPlan<N>::R1, R2 = TwoPlan<N>::R2;
     static constexpr bool EVEN = (32 % R1 == 0) && (32 % R2 == 0), WARP = EVEN || (R2 == 32 && R1 >= 24);
-    static constexpr int GR = EVEN ? 32 / R1 : WARP ? 1 : 128 / R2;
+    static constexpr int GR = EVEN ? 32 / (SPREAD ? (R1 > R2 ? R1 : R2) : R1) : WARP ? 1 : 128 / R2;
     static constexpr int GT = WARP ? 32 : (GR * R2 + 31) / 32 * 32;
     static constexpr int NT = WARP ? 128 : GT;
     static constexpr int LD = R1 | 1;  // odd: column walks of M touch every bank pair
@@ -62,11 +63,11 @@ template <int N> struct RowPlan {
     static constexpr size_t SMEM = (size_t)(N + NT / GT * GR * R2 * LD) * sizeof(float2);
 };
 
-template <int N>
-__global__ void __launch_bounds__(RowPlan<N>::NT, RowPlan<N>::BLOCKS)
+template <int N, bool SPREAD = false>
+__global__ void __launch_bounds__(RowPlan<N, SPREAD>::NT, RowPlan<N, SPREAD>::BLOCKS)
     two_rows(float2* __restrict__ psi, const float2* __restrict__ tmul, const float2* __restrict__ table, unsigned nx,
              FastDiv count, int inv, int fwd, float scale, const float2* const* __restrict__ t_of_wave) {
-    using P = RowPlan<N>;
+    using P = RowPlan<N, SPREAD>;
     constexpr int R1 = P::R1, R2 = P::R2, GT = P::GT, GR = P::GR, LD = P::LD, QA = P::QA, QB = P::QB;
     extern __shared__ __align__(16) float2 smem_two_rows[];
     float2* const tw = smem_two_rows;
@@ -488,24 +489,40 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
 }
 
 // ---- launches --------------------------------------------------------------------------------------------------------
-template <int N>
-bool launch_two_rows(Context& ctx, const float2* table, float2* psi, const float2* tmul, int nx, long long nrows, int inv,
-                     int fwd, float scale) {
-    using P = RowPlan<N>;
-    if (nrows >= (1LL << 31) - (1 << 20)) return false;
+template <int N, bool SPREAD>
+void launch_two_rows_s(Context& ctx, const float2* table, float2* psi, const float2* tmul, int nx, long long nrows, int inv,
+                       int fwd, float scale) {
+    using P = RowPlan<N, SPREAD>;
     static PerDevice setup;
     const int resident = setup.get([] {
-        allow_shared(two_rows<N>, P::SMEM);
+        allow_shared(two_rows<N, SPREAD>, P::SMEM);
         int n = 0;
-        SIMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, two_rows<N>, P::NT, P::SMEM));
+        SIMK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, two_rows<N, SPREAD>, P::NT, P::SMEM));
         return std::max(1, n);
     });
     const long long tiles = (nrows + P::GR - 1) / P::GR, per = P::NT / P::GT;
     const int grid = (int)std::min<long long>((tiles + per - 1) / per, (long long)resident * ctx.sm_count);
-    two_rows<N><<<grid, P::NT, P::SMEM, ctx.stream>>>(psi, tmul, table, (unsigned)nx, fast_div((unsigned)(nrows / nx)),
-                                                      inv, fwd, scale, ctx.wave_t);
+    two_rows<N, SPREAD><<<grid, P::NT, P::SMEM, ctx.stream>>>(psi, tmul, table, (unsigned)nx,
+                                                              fast_div((unsigned)(nrows / nx)), inv, fwd, scale,
+                                                              ctx.wave_t);
     SIMK_CUDA(cudaGetLastError());
     ++ctx.launches;
+}
+
+template <int N>
+bool launch_two_rows(Context& ctx, const float2* table, float2* psi, const float2* tmul, int nx, long long nrows, int inv,
+                     int fwd, float scale) {
+    if (nrows >= (1LL << 31) - (1 << 20)) return false;
+    // Up to four rows a multiprocessor (one 512^2 wave) a launch is one tile's chain of steps long: one row a warp is the
+    // shorter chain (512^2, one wave: 7.23 -> 6.90 us a pass, rows and columns; from two waves on no difference). Each row's
+    // arithmetic is the same.
+    if constexpr (RowPlan<N, true>::GR == 1 && RowPlan<N>::GR == 2) {
+        if (nrows <= 4LL * ctx.sm_count) {
+            launch_two_rows_s<N, true>(ctx, table, psi, tmul, nx, nrows, inv, fwd, scale);
+            return true;
+        }
+    }
+    launch_two_rows_s<N, false>(ctx, table, psi, tmul, nx, nrows, inv, fwd, scale);
     return true;
 }
 

@@ -274,12 +274,15 @@ __global__ void __launch_bounds__(256) k_poisson(const double* in, double* out, 
         if (tid < kPoissonBins) fill[tid] = 0;
         __syncthreads();
         int bin[kPoissonTile / 256];
+        double value[kPoissonTile / 256];  // all asked for before the first is used (no write may come between otherwise)
+#pragma unroll
+        for (int q = 0; q < kPoissonTile / 256; ++q) value[q] = tid + 256 * q < n ? in[first + tid + 256 * q] : 0.0;
 #pragma unroll
         for (int q = 0; q < kPoissonTile / 256; ++q) {
             const int i = tid + 256 * q;
             bin[q] = 0;
             if (i >= n) continue;
-            const double m = __dmul_rn(in[first + i], dose);
+            const double m = __dmul_rn(value[q], dose);
             if (!isfinite(m)) atomicOr(err, 2);
             const double lambda = (isfinite(m) && m > 0.0) ? m : 0.0;
             mean[i] = lambda;

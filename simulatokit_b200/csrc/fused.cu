@@ -1510,9 +1510,9 @@ bool cols_cc(Context& ctx, const RegPlan& p, const ColArgs& a, int count) {
 
 // ---- the two-pass engine (twopass.cuh): one exchange a transform, wherever the length has a plan and the settings ask
 // for no other engine. Measured against the engines it replaced (one box, us a launch, rows | columns, means over a
-// 6-slice scan's launches, probe generation and detection among the columns'): 512^2 x 512 waves 516 -> 420 | 488 -> 437;
-// 1024^2 x 128 671 -> 438 | 735 -> 544; 768^2 x 64 249 -> 148 | 246 -> 172; 500^2 x 144 691 -> 166 | 632 -> 167;
-// 256^2 x 256 69 -> 52 | 68 -> 60 -------------------------------------------------------------------------------------
+// 6-slice scan's launches, probe generation and detection among the columns'): 512^2 x 512 waves 516 -> 424 | 488 -> 443;
+// 1024^2 x 128 671 -> 441 | 735 -> 547; 768^2 x 64 249 -> 154 | 246 -> 176; 500^2 x 144 691 -> 161 | 632 -> 164;
+// 256^2 x 256 69 -> 54 | 68 -> 60 -------------------------------------------------------------------------------------
 bool two_wanted(const Context& ctx, int n) {
     if (!ctx.tma || !twopass_length(n)) return false;
     return comp_length(n) ? ctx.composite != 0 : true;

@@ -45,8 +45,8 @@ __device__ __forceinline__ unsigned operator/(unsigned n, const FastDiv& f) {
 }
 
 // ---- rows ------------------------------------------------------------------------------------------------------------
-// Bound by HBM where the DFTs are cheap (512: 5.1 TB/s of the measured 6.5, 420 us for 512 waves; 1024: 4.9), by issue
-// and the FMA pipe elsewhere (500 = 20 x 25: 3.5 TB/s, 166 us for 144 waves, FMA pipe near half busy).
+// Bound by HBM where the DFTs are cheap (512: 5.1 TB/s of the measured 6.5, 424 us for 512 waves; 1024: 4.9), by issue
+// and the FMA pipe elsewhere (500 = 20 x 25: 3.6 TB/s, 161 us for 144 waves, FMA pipe near half busy).
 // A group of GT threads takes GR rows at a time: one warp where R1 and R2 divide its lanes evenly (256, 512, 1024 and
 // 128 points: no barrier beyond __syncwarp), else a block.
 // SPREAD: at 512 a warp takes one row instead of two, half of step B's lanes idle, for launches of few rows.
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(RowPlan<N, SPREAD>::NT, RowPlan<N, SPREAD>::BL
 // and belongs to sub-block i % SUBS. TMA brings a tile in and takes it out; the load of tile i + NB is issued by the
 // sub-block that had tile i, once the store of tile i has read its buffer (asked for in the middle of its next tile).
 // Bound at 512 by the latency of a tile's three steps at four warps a scheduler (512 waves: 505 us between two slices,
-// 4.25 TB/s; 437 us the mean of a 6-slice scan's launches, as the times below; FMA pipe and issue near half busy).
+// 4.25 TB/s; 443 us the mean of a 6-slice scan's launches, as the times below; FMA pipe and issue near half busy).
 // Tiles loaded and stored from registers instead, without TMA: 541 us, most of it the loads' latency; tiles of 16
 // columns that way 550 us; P's first values asked for in step B 482 us, before the tile's wait 440 us. Programmatic
 // dependent launch of the passes cost 4 % at 512^2 (5 % at 256^2) and is not used.

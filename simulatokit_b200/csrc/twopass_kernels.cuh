@@ -235,6 +235,38 @@ template <int N> struct ColPlan {
     static constexpr size_t smem(int buffers) { return ((size_t)2 * N + (size_t)buffers * TILE) * sizeof(float2); }
 };
 
+// The wave's mean goes past the transforms of step B: it is taken off the R2 values of item 0 of line 0 beforehand, and
+// what P makes of it is added to them afterwards. A plane wave's energy is in that one value, and its rounding at each
+// level of the two transforms, slice after slice, was most of the error of sums over an exit wave (energy after 40 weak
+// slices, rms: 256^2 3.7e-7, now 4e-8; 640^2 4.1e-7, now 1.1e-7). One tile of a wave in ny / 8 has it. With R2 <= 16 the
+// item does this in registers; else in shared memory by functions of their own, as the registers of all items would be
+// planned for it (inlined: 512 446 -> 454 us, 640 105 -> 108; functions at 256 62.6 us, registers 60.8). It costs 2.5 % of
+// the pass at 256 (59.3 -> 60.8 us), 6 % at 576 (123 -> 131), elsewhere 1 % or less.
+// sum / R to 18 bits: R times that is exact (and only what is near the mean is needed: the rest stays in the values).
+template <int R> __device__ __forceinline__ float2 short_mean(float2 sum) {
+    static_assert(R <= 64, "18 bits and the radix's fit in 24");
+    return make_float2(__int_as_float(__float_as_int(sum.x * (1.0f / R)) & ~63),
+                       __int_as_float(__float_as_int(sum.y * (1.0f / R)) & ~63));
+}
+template <int R, int STEP> __device__ __noinline__ float2 take_mean(float2* x) {
+    float2 s = x[0];
+#pragma unroll 4
+    for (int j = 1; j < R; ++j) s = padd(s, x[j * STEP]);
+    s = short_mean<R>(s);
+#pragma unroll 4
+    for (int j = 0; j < R; ++j) x[j * STEP] = psub(x[j * STEP], s);
+    return s;
+}
+template <int R1, int R2, int STEP>
+__device__ __noinline__ void give_mean(float2* x, float2 z, const float2* tw_back, float scale, float rest) {
+    x[0] = make_float2(fmaf(z.x, scale, fmaf(z.x, rest, x[0].x)), fmaf(z.y, scale, fmaf(z.y, rest, x[0].y)));
+#pragma unroll 4
+    for (int j = 1; j < R2; ++j) {
+        const float s = tw_back[j * R1].x;
+        x[j * STEP] = make_float2(fmaf(z.x, s, x[j * STEP].x), fmaf(z.y, s, x[j * STEP].y));
+    }
+}
+
 struct TwoDetect {
     const int* ptr = nullptr;   // [groups C + 1]
     const int2* ent = nullptr;  // (row TC + column, weight bits)
@@ -262,6 +294,7 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
     extern __shared__ __align__(128) float2 smem_two_cols[];
     __shared__ __align__(8) uint64_t full[P::NB];
     __shared__ int failed[P::SUBS], issued[P::NB];
+    [[maybe_unused]] __shared__ float2 mean[P::SUBS];
     // W_N^{jk}, and for the way back the same divided by nx ny (so that scaling costs nothing: every value but j = 0
     // takes a twiddle)
     float2* const tw = smem_two_cols + buffers * TILE;
@@ -364,6 +397,8 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
                 issue(i - subs + buffers);
             }
         }
+        const bool zero = MODE == 0 && u == 0 && g == 0;  // has the wave's zero frequency
+        if (!SOON && zero) mean[sub] = take_mean<R2, TC>(M);
 #pragma unroll
         for (int q = 0; q < QB; ++q) {
             const int k = item + NT / TC * q, odd = SWAP ? (k & 1) : 0;
@@ -382,6 +417,15 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
                 if (EARLY > 0 && !SOON && q == 0) ask();
 #pragma unroll
                 for (int j = 0; j < R2; ++j) v[j] = j ? cmul(m[j & 1][j * TC], tw[j * R1 + k]) : m[0][0];
+                if (SOON && q == 0 && zero) {
+                    float2 s = v[0];
+#pragma unroll
+                    for (int j = 1; j < R2; ++j) s = padd(s, v[j]);
+                    s = short_mean<R2>(s);
+                    mean[sub] = s;
+#pragma unroll
+                    for (int j = 0; j < R2; ++j) v[j] = psub(v[j], s);
+                }
                 dft_reg<R2, -1>(v);
                 const float2* p = P0 + (size_t)(k + R1 * (q == 0 ? EARLY : 0)) * ny;
 #pragma unroll
@@ -396,6 +440,11 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
             }
             if constexpr (MODE == 0 || MODE == 2) {
                 dft_reg<R2, +1>(v);
+                if (SOON && q == 0 && zero) {
+                    const float2 z = cmul(make_float2(R2 * mean[sub].x, R2 * mean[sub].y), __ldg(P0));
+#pragma unroll
+                    for (int j = 0; j < R2; ++j) v[j] = padd(v[j], z);
+                }
 #pragma unroll
                 for (int j = 0; j < R2; ++j) {
                     // (j = 0 has no twiddle: scale + rest is 1 / (nx ny))
@@ -416,6 +465,8 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
                 }
             }
         }
+        if (!SOON && zero)
+            give_mean<R1, R2, TC>(M, cmul(make_float2(R2 * mean[sub].x, R2 * mean[sub].y), __ldg(P0)), tw_back, scale, rest);
         if constexpr (MODE == 1) fence_proxy_async_shared();
         group_sync<NT>(1 + sub);
         if constexpr (MODE == 0 || MODE == 2) {

@@ -47,3 +47,22 @@ def test_energy_of_jobs(n):
     table.add_probe(pot, sk.Probe(sk.ElectronBeam(200e3), pot.grid, sk.Aperture(20.0)), (7.3, 5.1))
     got = table.run()[0][0]
     assert abs(got.sum() / np.sum(np.abs(ref) ** 2) - 1) <= 1e-6
+
+
+@pytest.mark.parametrize("n", [200, 256, 500, 640])
+def test_energy_of_plane_waves(n):
+    """A plane wave's energy is in one value of its transform. Rounded to float32 once a slice, that would leave an error
+    of about 2^-24 sqrt(slices / 3) in the energy; it is less, as the transforms' levels don't round it one by one."""
+    slices, draws = 40, 6
+    grid = O.Grid(n, n, 0.061 * n, 0.061 * n)
+    errors = []
+    for draw in range(draws):
+        values = np.random.default_rng(1000 * n + draw).uniform(0, 30, (slices, n, n))
+        wave = np.ones((n, n), complex)
+        ref = O.multislice(wave, [O.transmission(v, 200e3, grid) for v in values], [2.0] * slices, 200e3, grid)[-1]
+        pot = sk.ProjectedPotential(sk.Grid(n, n, 0.061 * n, 0.061 * n), values, [2.0] * slices)
+        table = sk.JobTable()
+        table.add_plane_wave(pot, 200e3)
+        got = table.run()[0][0]
+        errors.append((got.sum() / got.size) / np.mean(np.abs(ref) ** 2) - 1)
+    assert np.sqrt(np.mean(np.square(errors))) <= 2.0 ** -24 * math.sqrt(slices / 3)

@@ -240,8 +240,8 @@ template <int N> struct ColPlan {
 // level of the two transforms, slice after slice, was most of the error of sums over an exit wave (energy after 40 weak
 // slices, rms: 256^2 3.7e-7, now 4e-8; 640^2 4.1e-7, now 1.1e-7). One tile of a wave in ny / 8 has it. With R2 <= 16 the
 // item does this in registers; else in shared memory by functions of their own, as the registers of all items would be
-// planned for it (inlined: 512 446 -> 454 us, 640 105 -> 108; functions at 256 62.6 us, registers 60.8). It costs 2.5 % of
-// the pass at 256 (59.3 -> 60.8 us), 6 % at 576 (123 -> 131), elsewhere 1 % or less.
+// planned for it (inlined: 512 446 -> 454 us, 640 105 -> 108; functions at 256 62.6 us, registers 60.5). It costs 2 % of
+// the pass at 256 (59.2 -> 60.5 us), 6 % at 576 (123 -> 131), elsewhere 1 % or less.
 // sum / R to 18 bits: R times that is exact (and only what is near the mean is needed: the rest stays in the values).
 template <int R> __device__ __forceinline__ float2 short_mean(float2 sum) {
     static_assert(R <= 64, "18 bits and the radix's fit in 24");
@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
 #pragma unroll
                     for (int j = 1; j < R2; ++j) s = padd(s, v[j]);
                     s = short_mean<R2>(s);
-                    mean[sub] = s;
+                    mean[sub] = cmul(make_float2(R2 * s.x, R2 * s.y), pe[0]);
 #pragma unroll
                     for (int j = 0; j < R2; ++j) v[j] = psub(v[j], s);
                 }
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(ColPlan<N>::NT* ColPlan<N>::SUBS, 1)
             if constexpr (MODE == 0 || MODE == 2) {
                 dft_reg<R2, +1>(v);
                 if (SOON && q == 0 && zero) {
-                    const float2 z = cmul(make_float2(R2 * mean[sub].x, R2 * mean[sub].y), __ldg(P0));
+                    const float2 z = mean[sub];
 #pragma unroll
                     for (int j = 0; j < R2; ++j) v[j] = padd(v[j], z);
                 }
